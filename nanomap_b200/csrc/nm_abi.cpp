@@ -530,6 +530,7 @@ int run_frame(nm_map m, nm_sensor s, nm::FrameParams& f, uint32_t flags, cudaStr
         if (ordered) {
           NM_CUDA(nm::tile_order_reserve(&m->tile_order, w.total_tiles, s0));
           w.order_scale = nm::tile_order_scale<1>(w);
+          w.split_bucket = nm::tile_split_bucket<1>(w);
           NM_CUDA(nm::launch_tile_order<1>(w, &m->tile_order, s0));
           w.order_counts = m->tile_order.counts;
           w.order_lists = m->tile_order.lists;
@@ -1149,6 +1150,7 @@ int nm_map_tick(nm_map m, const nm_frame* frames, int32_t n_frames, uint32_t fla
     if (!wide) {  // longest walks first
       NM_CUDA(nm::tile_order_reserve(&m->tile_order, w->total_tiles, s0));
       w->order_scale = nm::tile_order_scale<nm::kMaxTickFrames>(*w);
+      w->split_bucket = nm::tile_split_bucket<nm::kMaxTickFrames>(*w);
       NM_CUDA(nm::launch_tile_order<nm::kMaxTickFrames>(*w, &m->tile_order, s0));
       w->order_counts = m->tile_order.counts;
       w->order_lists = m->tile_order.lists;

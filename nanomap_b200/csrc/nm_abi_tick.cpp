@@ -184,6 +184,7 @@ int run_plan(nm_tick_plan p, uint32_t flags, cudaStream_t s) {
       w.order_lists = p->order.lists;
       w.order_cap = p->order.capacity;
       w.order_scale = nm::tile_order_scale<nm::kMaxTickFrames>(w);
+      w.split_bucket = nm::tile_split_bucket<nm::kMaxTickFrames>(w);
     }
   }
   if (m->view.capacity != p->captured_capacity || m->view.keys != p->captured_keys) {

@@ -111,6 +111,7 @@ struct TickWork {
   const uint32_t* order_lists;
   uint32_t order_cap;
   float order_scale;      // buckets per walk step: kOrderBuckets / (longest possible walk)
+  int32_t split_bucket;   // tiles of the buckets below this one are handed out in quarters
   uint32_t tile_start[MaxF + 1];
   int32_t tiles_x[MaxF];
   FrameParams fr[MaxF];
@@ -209,6 +210,9 @@ void tile_order_release(TileOrderBuffers* b);
 // kOrderBuckets / the longest walk any ray of these frames can take (steps + set-up).
 template <int MaxF>
 float tile_order_scale(const TickWork<MaxF>& w);
+// First bucket whose tiles are handed out whole (0: all are).
+template <int MaxF>
+int tile_split_bucket(const TickWork<MaxF>& w);
 // Files every tile under the bucket of its longest ray's walk (|R p|_1 / res, the DDA's step
 // count up to rounding, plus a set-up allowance).  The counts are zero on entry: the traversal
 // that reads a pass's lists clears them; `b.pending` (a pass whose traversal was never launched)

@@ -33,11 +33,6 @@ namespace {
 // than 16 x 16 on the headline frame)
 constexpr int kDepthTile = 8;
 
-struct LeafCache {
-  unsigned long long key;
-  int slot;
-};
-
 __device__ __forceinline__ void pixel_dir(const DepthParams& p, int w, int h, double d[3]) {
   double x, y, z;
   if (p.type == NM_SENSOR_FRUSTUM) {
@@ -71,13 +66,21 @@ __device__ __forceinline__ float seg_g(float u, float em1) {
   return (u * (1.0f + em1) + em1) / (u * u);
 }
 
+// expm1(-u), u >= 0.  A long ray runs through observed free space, where u is far below 2^-10 on
+// every lane of the warp and the series (next term u^4 / 24, below 1e-10 of u) replaces the
+// function, which is the longest part of a step's chain.
+__device__ __forceinline__ float expm1_neg(float u) {
+  if (u < 0x1p-10f) return -u * fmaf(u, fmaf(u, 1.0f / 6.0f, -0.5f), 1.0f);
+  return expm1f(-u);
+}
+
 // Every walk of a ray (forward, adjoint replays, refinement) ends where its transmittance
 // falls below this: what the rest of the ray could add to the expected depth is at most
 // kStopTransmittance x its remaining length (< 1e-6 voxel lengths for rays up to 1000
 // voxels), each such FP32 term being below half an ulp of the running integral once that
 // exceeds 0.01 voxels, and the rest's gradients carry the factor T too (there, the FP32 tail
-// A - P is rounding noise).  The three walks compute T with the same operations, so they
-// stop at the same voxel.
+// A - P is rounding noise).  The forward and the adjoint compute T with the same operations, so
+// they stop at the same voxel.
 constexpr float kStopTransmittance = 1e-9f;
 
 // Density of a log-odds value, memoised on the last value seen: along a ray most voxels share
@@ -87,6 +90,7 @@ struct DensityCache {
   bool has = false;
   float L = 0.0f;
   float sg = 0.0f, sig = 0.5f;
+  float inv = 0.0f;  // 1 / sg
   __device__ __forceinline__ void at(const DepthParams& p, float l) {
     if (!has || l != L) {
       has = true;
@@ -94,78 +98,125 @@ struct DensityCache {
       const float x = p.scale * l + p.bias;
       sg = softplus(x);
       sig = 1.0f / (1.0f + expf(-x));
+      inv = 1.0f / sg;
     }
+  }
+  // Integral of the transmittance over a segment of length D, em1 = expm1(-sg D).
+  __device__ __forceinline__ float segment(float em1, float D) const {
+    return sg > 0.0f ? -em1 * inv : D;
   }
 };
 
-// Visits the voxels of the ray after the start voxel: f(v, t_in, a_in, t_out, a_out), the
-// voxel entered at t_in < t_max across axis a_in and left at t_out = min(next crossing,
-// t_max) across a_out (-1 when clamped to t_max); f returns false to end the walk.  Crossings are (boundary - e) * (1 / d),
-// the reciprocal taken once per ray; per-axis state is kept in scalars (no local memory).
-template <class F>
-__device__ __forceinline__ void walk(const double e[3], const double d[3], double t_max, F&& f) {
-  int vx = (int)floor(e[0]), vy = (int)floor(e[1]), vz = (int)floor(e[2]);
+// Slot of a leaf in the map's table, or -1.  No depth kernel writes the table, so the keys may come
+// from L1 (neighbouring rays look the same leaves up).
+__device__ __forceinline__ int depth_find(const MapView& m, unsigned long long key) {
+  uint32_t h = hash_key(key) & m.mask;
+  const uint32_t limit = m.capacity < kMaxProbe ? m.capacity : kMaxProbe;
+  for (uint32_t probe = 0; probe < limit; ++probe) {
+    const unsigned long long k = __ldg(&m.keys[h]);
+    if (k == key) return (int)h;
+    if (k == kEmptyKey) return -1;
+    h = (h + 1) & m.mask;
+  }
+  return -1;
+}
+
+// Visits the voxels of the ray after the start voxel: f(slot, l, L, t_in, a_in, t_out), the voxel
+// (leaf slot or -1, index inside the leaf, log-odds) entered at t_in < t_max across axis a_in and
+// left at t_out = min(next crossing, t_max); f returns false to end the walk.  Crossings are
+// (boundary - e) * (1 / d), the reciprocal taken once per ray.
+//
+// A ray is a chain of steps, and a frame waits for its longest one (600 steps through observed free
+// space).  Ahead: the voxel after the current one is found, and its log-odds loaded, before the
+// current one is handed to f, so the load and the leaf look-up stay out of the chain (not for the
+// adjoint, whose gradient atomics bound it and whose registers are the tighter for it: 190 against
+// 185 us).  Times of one launch on the B200, before -> now: refinement step, 640x480 at 10 m and
+// 0.05 m, 140.5 -> 92 us, expected depth of
+// 1280x720 at 15 m and 0.02 m 872 -> 657 us, of 640x480 63.2 -> 56.6 us, its adjoint 185.8 -> 185.
+template <bool Ahead, class F>
+__device__ __forceinline__ void walk(const MapView& m, const float* __restrict__ vals,
+                                     const double e[3], const double d[3], double t_max, F&& f) {
+  const int vx = (int)floor(e[0]), vy = (int)floor(e[1]), vz = (int)floor(e[2]);
   const int sx = d[0] > 0.0 ? 1 : (d[0] < 0.0 ? -1 : 0);
   const int sy = d[1] > 0.0 ? 1 : (d[1] < 0.0 ? -1 : 0);
   const int sz = d[2] > 0.0 ? 1 : (d[2] < 0.0 ? -1 : 0);
   const double rx = sx ? __drcp_rn(d[0]) : 0.0;
   const double ry = sy ? __drcp_rn(d[1]) : 0.0;
   const double rz = sz ? __drcp_rn(d[2]) : 0.0;
-  auto cross = [](int v, int s, double e, double r) {
-    return __dmul_rn(__dadd_rn((double)(v + (s > 0 ? 1 : 0)), -e), r);
+  // next plane per axis, and the time of its crossing
+  int qx = vx + (sx > 0 ? 1 : 0), qy = vy + (sy > 0 ? 1 : 0), qz = vz + (sz > 0 ? 1 : 0);
+  double tx = sx ? __dmul_rn(__dadd_rn((double)qx, -e[0]), rx) : CUDART_INF;
+  double ty = sy ? __dmul_rn(__dadd_rn((double)qy, -e[1]), ry) : CUDART_INF;
+  double tz = sz ? __dmul_rn(__dadd_rn((double)qz, -e[2]), rz) : CUDART_INF;
+  int lx = vx >> 3, ly = vy >> 3, lz = vz >> 3;  // leaf of the voxel entered last
+  int l = local_index(vx, vy, vz);
+  int slot = depth_find(m, leaf_key(lx, ly, lz));
+  int a;  // axis crossed next
+  double t;
+  auto next = [&]() {
+    a = 2;
+    t = tz;
+    if (ty < t) {
+      a = 1;
+      t = ty;
+    }
+    if (tx < t) {
+      a = 0;
+      t = tx;
+    }
   };
-  double tx = sx ? cross(vx, sx, e[0], rx) : CUDART_INF;
-  double ty = sy ? cross(vy, sy, e[1], ry) : CUDART_INF;
-  double tz = sz ? cross(vz, sz, e[2], rz) : CUDART_INF;
-  int a_in = 2;
-  double t_in = tz;
-  if (ty < t_in) {
-    a_in = 1;
-    t_in = ty;
-  }
-  if (tx < t_in) {
-    a_in = 0;
-    t_in = tx;
-  }
-  const long long cap = 3ll * (long long)t_max + 16;
-  for (long long it = 0; it < cap && t_in < t_max; ++it) {
-    if (a_in == 0) {
-      vx += sx;
-      tx = cross(vx, sx, e[0], rx);
-    } else if (a_in == 1) {
-      vy += sy;
-      ty = cross(vy, sy, e[1], ry);
+  // enters the voxel across axis a: its leaf, index and log-odds
+  auto enter = [&]() -> float {
+    int msk, ds;
+    if (a == 0) {
+      qx += sx;
+      tx = __dmul_rn(__dadd_rn((double)qx, -e[0]), rx);
+      msk = 0x1C0;
+      ds = sx * 64;
+    } else if (a == 1) {
+      qy += sy;
+      ty = __dmul_rn(__dadd_rn((double)qy, -e[1]), ry);
+      msk = 0x38;
+      ds = sy * 8;
     } else {
-      vz += sz;
-      tz = cross(vz, sz, e[2], rz);
+      qz += sz;
+      tz = __dmul_rn(__dadd_rn((double)qz, -e[2]), rz);
+      msk = 0x7;
+      ds = sz;
     }
-    int a_out = 2;
-    double t_out = tz;
-    if (ty < t_out) {
-      a_out = 1;
-      t_out = ty;
+    const int vv = (l & msk) + ds;
+    l = (l & ~msk) | (vv & msk);
+    if ((unsigned)vv > (unsigned)msk) {
+      lx += a == 0 ? sx : 0;
+      ly += a == 1 ? sy : 0;
+      lz += a == 2 ? sz : 0;
+      slot = depth_find(m, leaf_key(lx, ly, lz));
     }
-    if (tx < t_out) {
-      a_out = 0;
-      t_out = tx;
+    return slot >= 0 ? __ldg(&vals[(size_t)slot * kLeafVoxels + l]) : 0.0f;
+  };
+  next();
+  if (!(t < t_max)) return;
+  const long long cap = 3ll * (long long)t_max + 16;
+  if (Ahead) {
+    float L = enter();
+    for (long long it = 0; it < cap; ++it) {
+      const int slot0 = slot, l0 = l, a_in = a;
+      const double t_in = t;
+      const float L0 = L;
+      next();
+      const bool more = t < t_max;
+      if (more) L = enter();
+      if (!f(slot0, l0, L0, t_in, a_in, more ? t : t_max) || !more) break;
     }
-    const int v[3] = {vx, vy, vz};
-    if (!(t_out < t_max ? f(v, t_in, a_in, t_out, a_out) : f(v, t_in, a_in, t_max, -1))) break;
-    a_in = a_out;
-    t_in = t_out;
+  } else {
+    for (long long it = 0; it < cap && t < t_max; ++it) {
+      const float L = enter();
+      const int a_in = a;
+      const double t_in = t;
+      next();
+      if (!f(slot, l, L, t_in, a_in, t < t_max ? t : t_max)) break;
+    }
   }
-}
-
-__device__ __forceinline__ float voxel_logodds(const MapView& m, const float* vals, LeafCache& c,
-                                               const int v[3], int* slot, int* l) {
-  const unsigned long long key = leaf_key(v[0] >> 3, v[1] >> 3, v[2] >> 3);
-  if (key != c.key) {
-    c.key = key;
-    c.slot = map_find(m, key);
-  }
-  *slot = c.slot;
-  *l = local_index(v[0], v[1], v[2]);
-  return c.slot >= 0 ? __ldg(&vals[(size_t)c.slot * kLeafVoxels + *l]) : 0.0f;
 }
 
 // Expected depth in index units (integral of the transmittance over [0, t_max]), FP32.  With
@@ -176,7 +227,6 @@ __device__ __forceinline__ float expected_index_depth(const DepthParams& p, cons
                                                       const float* vals, const double d[3],
                                                       float* t1_out, uint32_t* visits,
                                                       float* entry_step = nullptr) {
-  LeafCache c{kEmptyKey, -1};
   DensityCache dc;
   float T = 1.0f, acc = 0.0f, W = 0.0f;
   double t1 = p.t_max;
@@ -184,18 +234,17 @@ __device__ __forceinline__ float expected_index_depth(const DepthParams& p, cons
   uint32_t n = 0;
   const float step[3] = {(float)(1.0 / fabs(d[0])), (float)(1.0 / fabs(d[1])),
                          (float)(1.0 / fabs(d[2]))};
-  walk(p.eye, d, p.t_max, [&](const int v[3], double t_in, int a_in, double t_out, int) {
+  walk<true>(m, vals, p.eye, d, p.t_max, [&](int, int, float L, double t_in, int a_in, double t_out) {
     ++n;
-    int slot, l;
-    dc.at(p, voxel_logodds(m, vals, c, v, &slot, &l));
+    dc.at(p, L);
     const float sg = dc.sg;
     const float Dk = (float)(t_out - t_in);
     if (first) {
       t1 = t_in;
       first = false;
     }
-    const float em1 = expm1f(-sg * Dk);
-    acc += T * (sg > 0.0f ? -em1 / sg : Dk);
+    const float em1 = expm1_neg(sg * Dk);
+    acc += T * dc.segment(em1, Dk);
     if (entry_step) W -= T * em1 * step[a_in];
     T *= 1.0f + em1;
     return T >= kStopTransmittance;
@@ -257,7 +306,6 @@ __device__ __forceinline__ void replay_gradients(const DepthParams& p, const Map
                                                  const float* vals, const double d[3], float D,
                                                  float t1, float gd, float* grad_vals,
                                                  float g6[6], uint32_t* visits) {
-  LeafCache c{kEmptyKey, -1};
   DensityCache dc;
   uint32_t n = 0;
   float T = 1.0f, P = 0.0f, sg_prev = 0.0f;
@@ -265,9 +313,8 @@ __device__ __forceinline__ void replay_gradients(const DepthParams& p, const Map
   const float inv_d[3] = {(float)(1.0 / d[0]), (float)(1.0 / d[1]), (float)(1.0 / d[2])};
   const float gv = gd * (float)p.res * p.scale;
   const float tail0 = D - t1;
-  walk(p.eye, d, p.t_max, [&](const int v[3], double t_in, int a_in, double t_out, int) {
-    int slot, l;
-    dc.at(p, voxel_logodds(m, vals, c, v, &slot, &l));
+  walk<false>(m, vals, p.eye, d, p.t_max, [&](int slot, int l, float L, double t_in, int a_in, double t_out) {
+    dc.at(p, L);
     ++n;
     const float sg = dc.sg;
     const float Dk = (float)(t_out - t_in);
@@ -285,8 +332,8 @@ __device__ __forceinline__ void replay_gradients(const DepthParams& p, const Map
       gdir[2] -= gc * ti;
     }
     const float u = sg * Dk;
-    const float em1 = expm1f(-u);
-    const float Pn = P + T * (sg > 0.0f ? -em1 / sg : Dk);
+    const float em1 = expm1_neg(u);
+    const float Pn = P + T * dc.segment(em1, Dk);
     if (grad_vals) {
       const float dsig = T * Dk * Dk * seg_g(u, em1) - Dk * (tail0 - Pn);
       if (t_in < kGatherSpan)
@@ -357,8 +404,9 @@ __global__ void __launch_bounds__(kDepthTile * kDepthTile) k_depth_forward(Depth
 }
 
 // `depth` (may be null): the forward's output at this pose and these values; the ray's
-// expected depth is then taken from it instead of a first replay.
-__global__ void __launch_bounds__(kDepthTile * kDepthTile) k_depth_backward(
+// expected depth is then taken from it instead of a first replay.  16 CTAs per SM (64 registers): 185
+// us for a 640x480 adjoint given depths; 195 us at 79 registers.
+__global__ void __launch_bounds__(kDepthTile * kDepthTile, 16) k_depth_backward(
     DepthParams p, MapView m, const float* vals, const float* grad_depth, const float* depth,
     float* grad_vals, double* partials) {
   const int w = blockIdx.x * kDepthTile + threadIdx.x;
@@ -398,7 +446,6 @@ __device__ __forceinline__ float depth_and_pose_gradient(const DepthParams& p, c
                                                          const float* vals, const double d[3],
                                                          uint32_t* visits, float* entry_step,
                                                          float g6[6]) {
-  LeafCache c{kEmptyKey, -1};
   DensityCache dc;
   float T = 1.0f, acc = 0.0f, W = 0.0f, sg_prev = 0.0f;
   double t1 = p.t_max;
@@ -409,10 +456,9 @@ __device__ __forceinline__ float depth_and_pose_gradient(const DepthParams& p, c
   const float inv_d[3] = {(float)(1.0 / d[0]), (float)(1.0 / d[1]), (float)(1.0 / d[2])};
   double sc[3] = {0.0, 0.0, 0.0}, scp[3] = {0.0, 0.0, 0.0};
   double sct[3] = {0.0, 0.0, 0.0}, sctp[3] = {0.0, 0.0, 0.0};
-  walk(p.eye, d, p.t_max, [&](const int v[3], double t_in, int a_in, double t_out, int) {
+  walk<true>(m, vals, p.eye, d, p.t_max, [&](int, int, float L, double t_in, int a_in, double t_out) {
     ++n;
-    int slot, l;
-    dc.at(p, voxel_logodds(m, vals, c, v, &slot, &l));
+    dc.at(p, L);
     const float sg = dc.sg;
     const float Dk = (float)(t_out - t_in);
     if (first) {
@@ -439,7 +485,10 @@ __device__ __forceinline__ float depth_and_pose_gradient(const DepthParams& p, c
         sctp[2] += cd * ti * P;
       }
     }
-    const float em1 = expm1f(-sg * Dk);
+    // The refinement's path doubles differences of rounding from step to step, so the segment's
+    // integral keeps the division and the function; -u is expm1f(-u)'s own value for u this small.
+    const float u = sg * Dk;
+    const float em1 = u < 0x1p-26f ? -u : expm1f(-u);
     acc += T * (sg > 0.0f ? -em1 / sg : Dk);
     W -= T * em1 * step[a_in];
     T *= 1.0f + em1;
@@ -543,68 +592,97 @@ __device__ void rotate_left(const double phi[3], double R[9]) {
   for (int i = 0; i < 9; ++i) R[i] = out[i];
 }
 
-// One block: the step's partials summed in a fixed order (loss, count, 6 gradients), then
-// thread 0 records the mean loss and, before the last step, applies Adam on the left
-// world-frame increment (rho, phi) with the learning rates cosine-decayed to zero.
-__global__ void k_refine_update(const double* partials, int n, RefineState* st, float* losses,
-                                int it) {
-  __shared__ double s[256];
-  __shared__ double h[8];
-  for (int c = 0; c < 8; ++c) {
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) acc += partials[(size_t)i * 8 + c];
-    s[threadIdx.x] = acc;
-    __syncthreads();
-    for (int k = blockDim.x / 2; k > 0; k >>= 1) {
-      if ((int)threadIdx.x < k) s[threadIdx.x] += s[threadIdx.x + k];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) h[c] = s[0];
-    __syncthreads();
+// Column sums of an (n, N) array of partials, N <= 8, by one block of kSumThreads threads in a
+// fixed order (deterministic); h[c] = sum of column c, on every thread.  Thread t adds rows t / 8,
+// t / 8 + 128, ... of column t % 8 (neighbouring threads read neighbouring words, four rows in
+// flight), then a shuffle tree and one over the warps.  Bound by the latency of its 10 dependent
+// loads: 40.7 -> 9 us in the refinement step's update and 27.7 -> 6 us after an adjoint, both for
+// the 4800 rows of a 640x480 image (one column at a time over 256 threads before).
+constexpr int kSumThreads = 1024;
+template <int N>
+__device__ __forceinline__ void column_sums(const double* __restrict__ partials, int n, double h[N]) {
+  __shared__ double s[kSumThreads / 32][8];
+  const int c = threadIdx.x & 7, r0 = threadIdx.x >> 3;
+  constexpr int kRows = kSumThreads / 8;
+  double x[4] = {0.0, 0.0, 0.0, 0.0};
+  if (c < N) {
+    int i = r0;
+    for (; i + 3 * kRows < n; i += 4 * kRows)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[k] += partials[(size_t)(i + k * kRows) * N + c];
+    for (int k = 0; i < n; i += kRows, ++k) x[k] += partials[(size_t)i * N + c];
   }
-  if (threadIdx.x != 0 || st->error) return;
+  double sum = (x[0] + x[1]) + (x[2] + x[3]);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+  if ((threadIdx.x & 31) < 8) s[threadIdx.x >> 5][c] = sum;
+  __syncthreads();
+  if (threadIdx.x < 32) {  // 4 warps' sums a lane, then the four lanes of a column
+    double y = 0.0;
+#pragma unroll
+    for (int k = 0; k < kSumThreads / 128; ++k) y += s[(threadIdx.x >> 3) + 4 * k][c];
+    y += __shfl_xor_sync(0xffffffffu, y, 8);
+    y += __shfl_xor_sync(0xffffffffu, y, 16);
+    if (threadIdx.x < 8) s[0][c] = y;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < N; ++k) h[k] = s[0][k];
+}
+
+// One block: the step's partials summed in a fixed order (loss, count, 6 gradients), then
+// the mean loss is recorded and, before the last step, Adam is applied on the left world-frame
+// increment (rho, phi), a component per lane, with the learning rates cosine-decayed to zero.
+__global__ void __launch_bounds__(kSumThreads) k_refine_update(const double* partials, int n,
+                                                               RefineState* st, float* losses,
+                                                               int it) {
+  double h[8];
+  column_sums<8>(partials, n, h);
+  if (threadIdx.x >= 32 || st->error) return;
   if (h[1] < 1.0) {
-    st->error |= kRefineNoPixels;
+    if (threadIdx.x == 0) st->error |= kRefineNoPixels;
     return;
   }
-  losses[it] = (float)(h[0] / h[1]);
+  if (threadIdx.x == 0) losses[it] = (float)(h[0] / h[1]);
   if (it >= st->steps) return;
   const double b1 = 0.9, b2 = 0.999, eps = 1e-8;
   const double t = (double)(it + 1);
-  const double decay = 0.5 * (1.0 + cos(CUDART_PI * it / st->steps));
-  double step[6];
-  for (int i = 0; i < 6; ++i) {
-    const double g = h[2 + i] / h[1];
-    st->mom[i] = b1 * st->mom[i] + (1.0 - b1) * g;
-    st->var[i] = b2 * st->var[i] + (1.0 - b2) * g * g;
-    const double mh = st->mom[i] / (1.0 - pow(b1, t));
-    const double vh = st->var[i] / (1.0 - pow(b2, t));
-    step[i] = -decay * (i < 3 ? st->lr_position : st->lr_rotation) * mh / (sqrt(vh) + eps);
+  double step = 0.0;
+  const int i = threadIdx.x;
+  if (i < 6) {
+    const double decay = 0.5 * (1.0 + cos(CUDART_PI * it / st->steps));
+    double gi = h[2];
+#pragma unroll
+    for (int k = 1; k < 6; ++k) gi = i == k ? h[2 + k] : gi;
+    const double g = gi / h[1];
+    const double mom = b1 * st->mom[i] + (1.0 - b1) * g;
+    const double var = b2 * st->var[i] + (1.0 - b2) * g * g;
+    st->mom[i] = mom;
+    st->var[i] = var;
+    const double mh = mom / (1.0 - pow(b1, t));
+    const double vh = var / (1.0 - pow(b2, t));
+    step = -decay * (i < 3 ? st->lr_position : st->lr_rotation) * mh / (sqrt(vh) + eps);
   }
-  for (int a = 0; a < 3; ++a)
-    if (fabs((st->position[a] + step[a]) / st->res) + st->t_max + 2.0 > (double)(1 << 23) - 16.0) {
-      st->error |= kRefineOutOfRange;
-      return;
-    }
-  for (int a = 0; a < 3; ++a) st->position[a] += step[a];
-  rotate_left(step + 3, st->R);
+  const bool out = i < 3 && fabs((st->position[i < 3 ? i : 0] + step) / st->res) + st->t_max + 2.0 >
+                                (double)(1 << 23) - 16.0;
+  if (__any_sync(0xffffffffu, out)) {
+    if (i == 0) st->error |= kRefineOutOfRange;
+    return;
+  }
+  if (i < 3) st->position[i] += step;
+  double phi[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) phi[k] = __shfl_sync(0xffffffffu, step, 3 + k);
+  if (i == 0) rotate_left(phi, st->R);
 }
 
-// Column sums of an (n, N) array of partials in a fixed order (deterministic).
-__global__ void k_sum_partials(const double* partials, int n, int N, double* out) {
-  __shared__ double s[256];
-  for (int c = 0; c < N; ++c) {
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) acc += partials[(size_t)i * N + c];
-    s[threadIdx.x] = acc;
-    __syncthreads();
-    for (int k = blockDim.x / 2; k > 0; k >>= 1) {
-      if ((int)threadIdx.x < k) s[threadIdx.x] += s[threadIdx.x + k];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) out[c] = s[0];
-    __syncthreads();
-  }
+__global__ void __launch_bounds__(kSumThreads) k_sum_partials(const double* partials, int n,
+                                                              double* out) {
+  double h[6];
+  column_sums<6>(partials, n, h);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int c = 0; c < 6; ++c) out[c] = h[c];
 }
 
 dim3 depth_grid(const DepthParams& p) {
@@ -632,7 +710,7 @@ cudaError_t launch_depth_backward(const DepthParams& p, const MapView& m, const 
                                                               grad_vals, partials);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_sum_partials<<<1, 256, 0, s>>>(partials, (int)(g.x * g.y), 6, out6);
+  k_sum_partials<<<1, kSumThreads, 0, s>>>(partials, (int)(g.x * g.y), out6);
   return cudaGetLastError();
 }
 
@@ -645,7 +723,7 @@ cudaError_t launch_depth_refine(const DepthParams& p, const MapView& m, const fl
                                                             surface_offset, edge, st, partials);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_refine_update<<<1, 256, 0, s>>>(partials, (int)(g.x * g.y), st, losses, it);
+  k_refine_update<<<1, kSumThreads, 0, s>>>(partials, (int)(g.x * g.y), st, losses, it);
   return cudaGetLastError();
 }
 

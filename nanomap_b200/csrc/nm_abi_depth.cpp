@@ -113,6 +113,14 @@ int nm_map_values_copy(nm_map m, float* dst, uint64_t max_floats, uint64_t* n_fl
   if (max_floats < n) return fail(NM_ERR_ARG, "destination holds %llu floats, map needs %llu",
                                   (unsigned long long)max_floats, (unsigned long long)n);
   NM_CUDA(cudaSetDevice(m->ctx->device));
+  // this device's aligned memory takes the kernel that does not read empty slots
+  cudaPointerAttributes at{};
+  if (((uintptr_t)dst & 15u) == 0 && cudaPointerGetAttributes(&at, dst) == cudaSuccess &&
+      at.type == cudaMemoryTypeDevice && at.device == m->ctx->device) {
+    NM_CUDA(nm::launch_values_copy(m->view, dst, m->ctx->sm_count, nm::pick(m->ctx, stream)));
+    return NM_OK;
+  }
+  cudaGetLastError();
   NM_CUDA(cudaMemcpyAsync(dst, m->view.values, n * sizeof(float), cudaMemcpyDeviceToDevice,
                           nm::pick(m->ctx, stream)));
   return NM_OK;

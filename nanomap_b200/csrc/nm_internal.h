@@ -240,6 +240,8 @@ cudaError_t launch_rehash(const MapView& from, const MapView& to, uint32_t cur_e
                           int update_mode, cudaStream_t s);
 cudaError_t launch_export(const MapView& m, int32_t* origins, float* values, uint32_t* active,
                           uint32_t* n_out, uint32_t max_out, cudaStream_t s);
+// All slots' log-odds to `dst` (device memory, 16-byte aligned).
+cudaError_t launch_values_copy(const MapView& m, float* dst, int sm_count, cudaStream_t s);
 cudaError_t launch_export_labels(const MapView& m, int plane, int32_t* origins,
                                  uint32_t* words, uint32_t* n_out, uint32_t max_out,
                                  cudaStream_t s);

@@ -73,13 +73,21 @@ __device__ __forceinline__ int sim_level(const SimMapView& v, int x, int y, int 
 
 // Distance (metres) to the first active voxel entered along the ray from `eye` (index space)
 // in the unit direction `dir`, at a ray time within [tmin, tmax] (voxel units), or 0.  The
-// voxel holding the eye is not tested.
+// voxel holding the eye is not tested.  With nseg > 1 the walk covers only the seg-th of nseg parts of
+// the ray: the voxels entered in (start, end] of the part.  Crossing times have no accumulated state,
+// so the voxel that the whole walk is in at the part's start is found directly: on each axis it
+// has crossed every plane whose time is not above the start.  *found: an active voxel ended the walk
+// (also one whose distance is 0).
 __device__ __forceinline__ float sim_cast(const SimMapView& v, const float eye[3], float dir[3],
-                                          float tmin, float tmax) {
+                                          float tmin, float tmax, int seg = 0, int nseg = 1,
+                                          bool* found = nullptr) {
   float result = 0.0f;
   float inv[3];
   int st[3];
-  float t_in = 0.0f, t_out = INFINITY;
+  // Nothing past tmax can be a result, so the walk ends there and not only where the ray leaves the
+  // map (a NaN tmax leaves it the map's end): 512 rays of 5 m in a 20 m world 94 -> 62 us, a frame
+  // whose rays mostly end on something 64.2 -> 63.2 us.
+  float t_in = 0.0f, t_out = fminf(INFINITY, tmax);
   bool miss = false;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
@@ -107,6 +115,21 @@ __device__ __forceinline__ float sim_cast(const SimMapView& v, const float eye[3
 #pragma unroll
     for (int a = 0; a < 3; ++a) k[a] = (int)floorf(__fadd_rn(eye[a], __fmul_rn(dir[a], t_in)));
     float t = t_in;
+    if (nseg > 1 && !(t_out < 1e6f)) {  // no end to divide: the first lane takes the whole ray
+      if (seg > 0) return 0.0f;
+    } else if (nseg > 1) {
+      const float part = __fdiv_rn(__fadd_rn(t_out, -t_in), (float)nseg);
+      const float t0 = __fadd_rn(t_in, __fmul_rn(part, (float)seg));
+      // (the parts' ends do not fall with seg, and neighbours compute the same value)
+      if (seg + 1 < nseg) t_out = fminf(t_out, __fadd_rn(t_in, __fmul_rn(part, (float)(seg + 1))));
+      if (seg > 0) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          if (st[a] != 0)
+            k[a] = advance_axis(k[a], k[a] + st[a] * (1 << 22), st[a], eye[a], dir[a], inv[a], t0, true);
+        t = t0;
+      }
+    }
     bool first = true;
     for (int iter = 0; iter < (1 << 22); ++iter) {
       int leaf = -1;
@@ -158,6 +181,7 @@ __device__ __forceinline__ float sim_cast(const SimMapView& v, const float eye[3
         k[1] = k1;
         k[2] = k2;
         if (hit) {
+          if (found) *found = true;
           if (t >= tmin && t <= tmax) result = __fmul_rn(t, v.res);
           break;
         }

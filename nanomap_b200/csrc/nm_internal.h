@@ -165,8 +165,7 @@ struct FilterBuffers {
   uint32_t* out_counts;            // compact: input points per filtered point
   float* idx_pts;                  // by input index: 3 floats at the voxel's first point
   uint32_t* idx_tags;              // by input index: tag of the frame that wrote idx_pts
-  float* dense_pts;                // tagged idx_pts packed in input order
-  uint32_t* block_counts;          // compaction: tagged indices per block, then their prefix
+  float* dense_pts;                // tagged idx_pts packed, 1024 positions at a time
   uint32_t* n_dense;               // device count of dense points
   int64_t capacity;
   uint32_t table_mask;

@@ -1757,7 +1757,9 @@ int tile_split_bucket(const TickWork<MaxF>& w) {
   const int quarter = w.tile_w * w.tile_h / 4;
   if ((w.tile_w & 15) != 0 || (w.tile_h & 7) != 0 || (quarter > kMarchRays && quarter % kMarchRays != 0))
     return 0;
-  const float steps = std::max(96.0f, kSplitSteps + kSplitStepsPerTile * (float)w.total_tiles);
+  // (of a filtered frame's tiles only the first few hold points, how many the device knows)
+  const float tiles = w.fr[0].input_kind == 2 ? 0.0f : (float)w.total_tiles;
+  const float steps = std::max(96.0f, kSplitSteps + kSplitStepsPerTile * tiles);
   const float q = steps * w.order_scale;
   return q < (float)kOrderBuckets ? kOrderBuckets - (int)q : 0;
 }

@@ -285,10 +285,24 @@ uint64_t frame_leaf_bound(nm_map m, nm_sensor s, const nm_pose& pose, const floa
   return (uint64_t)std::min(box_leaves(lo, hi), ray_leaf_cap(m, s, n_rays));
 }
 
-int ensure_capacity(nm_map m, uint64_t bound, cudaStream_t s) {
-  const uint64_t limit = m->view.capacity / 2;
-  if (m->known_leaves + m->pending_bound + bound <= limit) {
-    m->pending_bound += bound;
+// Leaves that a frame of this sensor can touch at most, wherever it looks: leaves are disjoint, and
+// those that meet the ball of its range lie in the ball widened by a leaf's diagonal.
+double ball_leaves(nm_map m, nm_sensor s) {
+  const double r = (s->desc.max_range / m->desc.res + 2.0) / 8.0 + 1.7320509;
+  return 4.1887903 * r * r * r;
+}
+
+// Room for a frame that touches up to `bound` leaves (the measure the table grows by) and for certain
+// no more than `most` (<= bound).  The leaf count is read, waiting for the stream, only when the
+// frames since the last read could together pass 7/8 of the table, short of which probing ends well
+// inside its limit; the table still grows as soon as a count read finds the frame's bound not to
+// fit in half of it.  With a wait whenever the bounds passed one half, xyz records at 10 m and 0.05 m
+// (137 K leaves a bound, 82 K in the ball) waited every frame in a table of 2^19 slots: 16 frames
+// 2037 -> 1805 us, voxel-filtered 2350 -> 2118 us.
+int ensure_capacity(nm_map m, uint64_t bound, uint64_t most, cudaStream_t s) {
+  const uint64_t limit = m->view.capacity / 2, full = (uint64_t)m->view.capacity / 8 * 7;
+  if (m->known_leaves + bound <= limit && m->known_leaves + m->pending_bound + most <= full) {
+    m->pending_bound += most;
     return NM_OK;
   }
   NM_CUDA(cudaStreamSynchronize(s));
@@ -305,7 +319,7 @@ int ensure_capacity(nm_map m, uint64_t bound, cudaStream_t s) {
     const int rc = grow_map(m, (uint32_t)cap, s);
     if (rc != NM_OK) return rc;
   }
-  m->pending_bound = bound;
+  m->pending_bound = most;
   return NM_OK;
 }
 
@@ -493,7 +507,7 @@ int apply_filter(nm_map m, nm::FrameParams& f, uint32_t flags, cudaStream_t s0) 
 
 int run_frame(nm_map m, nm_sensor s, nm::FrameParams& f, uint32_t flags, cudaStream_t s0,
               uint64_t bound, const nm::SimRender* sim) {
-  int rc = ensure_capacity(m, bound, s0);
+  int rc = ensure_capacity(m, bound, (uint64_t)std::min((double)bound, ball_leaves(m, s)), s0);
   if (rc != NM_OK) return rc;
   rc = set_plane_constants(m, 0, s);
   if (rc != NM_OK) return rc;
@@ -1141,7 +1155,7 @@ int nm_map_tick(nm_map m, const nm_frame* frames, int32_t n_frames, uint32_t fla
   }
   bound = (uint64_t)std::min(box_leaves(ulo, uhi), cap);
   w->total_tiles = w->tile_start[n_frames];
-  int rc = ensure_capacity(m, bound, s0);
+  int rc = ensure_capacity(m, bound, bound, s0);
   if (rc != NM_OK) return rc;
   for (int i = 0; i < n_frames; ++i) w->fr[i].epoch = m->epoch;
   if (w->total_tiles > 0) {

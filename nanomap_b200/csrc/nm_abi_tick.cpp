@@ -166,7 +166,7 @@ int run_plan(nm_tick_plan p, uint32_t flags, cudaStream_t s) {
   uint64_t bound = 0;
   int rc = fill_stage(p, p->h_stage[k], &bound);
   if (rc != NM_OK) return rc;
-  rc = nm::ensure_capacity(m, bound, s);
+  rc = nm::ensure_capacity(m, bound, bound, s);
   if (rc != NM_OK) return rc;
   const uint32_t tiles = p->h_stage[k]->work.total_tiles;
   if (tiles > p->order.capacity) {  // the graphs hold the buffers' addresses

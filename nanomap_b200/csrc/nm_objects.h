@@ -136,7 +136,7 @@ void frame_box(nm_map m, nm_sensor s, const nm_pose& pose, const float R[9], boo
                double lo[3], double hi[3]);
 double box_leaves(const double lo[3], const double hi[3]);
 double ray_leaf_cap(nm_map m, nm_sensor s, uint64_t n_rays);
-int ensure_capacity(nm_map m, uint64_t bound, cudaStream_t s);
+int ensure_capacity(nm_map m, uint64_t bound, uint64_t most, cudaStream_t s);
 int set_plane_constants(nm_map m, int plane, nm_sensor s);
 IntegrateParams integrate_params(nm_map m);
 // `dependent`: the last operation on `s` is a traversal kernel, so the integration may be

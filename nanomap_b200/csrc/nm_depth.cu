@@ -131,7 +131,7 @@ __device__ __forceinline__ int depth_find(const MapView& m, unsigned long long k
 // current one is handed to f, so the load and the leaf look-up stay out of the chain (not for the
 // adjoint, whose gradient atomics bound it and whose registers are the tighter for it: 190 against
 // 185 us).  Times of one launch on the B200, before -> now: refinement step, 640x480 at 10 m and
-// 0.05 m, 140.5 -> 92 us, expected depth of
+// 0.05 m, 140.5 -> 92 us (85 with kRefineBlocks), expected depth of
 // 1280x720 at 15 m and 0.02 m 872 -> 657 us, of 640x480 63.2 -> 56.6 us, its adjoint 185.8 -> 185.
 template <bool Ahead, class F>
 __device__ __forceinline__ void walk(const MapView& m, const float* __restrict__ vals,
@@ -537,7 +537,12 @@ __device__ __forceinline__ bool target_edge(const float* target, int W, int H, i
 // surface at the face the ray enters; 0.5: at the middle of the voxel), the offset held fixed
 // for the gradient.  Silhouette pixels of the target are left out when edge > 0.  Partials:
 // loss, count, 6 gradients.
-__global__ void __launch_bounds__(kDepthTile * kDepthTile) k_depth_refine(
+//
+// A chain of steps per ray, so the blocks resident set the rate: 8 per SM (115 registers) 92 us for 640x480
+// at 10 m and 0.05 m, 10 (96) 88, 12 (80, with spills) 85, 14 84, 16 (64) 85.
+// (The forward kernel has 18 without a limit and the adjoint 16: more of them only spilled.)
+constexpr int kRefineBlocks = 12;
+__global__ void __launch_bounds__(kDepthTile * kDepthTile, kRefineBlocks) k_depth_refine(
     DepthParams p0, MapView m, const float* vals, const float* target, float max_residual,
     float surface_offset, float edge, const RefineState* st, double* partials) {
   // the pose of this step, from the device state (the eye as the host computes it)

@@ -1401,8 +1401,12 @@ __device__ __forceinline__ void tile_order_body(const TickWork<MaxF>& work, Tile
   const uint32_t tile = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31;
   const int nrays = work.tile_w * work.tile_h;
-  int fi = 0;
-  while (fi + 1 < work.n_frames && work.tile_start[fi + 1] <= tile) ++fi;
+  // the tile's frame, every start read at once: one after the other they were most of a CTA's time
+  // (16-frame tick, 20 K tiles: 38.7 -> 30 us)
+  static_assert(MaxF <= 32, "a lane per frame");
+  const int fi = MaxF == 1 ? 0
+                           : __popc(__ballot_sync(kFull, lane > 0 && lane < work.n_frames &&
+                                                             work.tile_start[lane < MaxF ? lane : 0] <= tile));
   const FrameParams& f = work.fr[fi];
   const uint32_t lt = tile - work.tile_start[fi];
   const int x0 = (int)(lt % (uint32_t)work.tiles_x[fi]) * work.tile_w;

@@ -1559,12 +1559,15 @@ constexpr int kCountLeafWords = kLeafVoxels / 4;       // voxel l: byte l >> 7 o
                                                        // neighbours lie in different words
 constexpr size_t kCountBytes = (size_t)kCountLeaves * kCountLeafWords * 4;
 
+// A leaf that the walk has entered and not looked up.  (No entry, slot or lost leaf has this number.)
+constexpr int kNoEntry = INT_MIN + 1;
+
 __device__ __forceinline__ uint32_t count_home(uint32_t code) {
   return __umulhi(code * 0x9E3779B1u, (uint32_t)kCountLeaves);
 }
 
-// Entry of a leaf, or -(g + 1) for slot g of the device table where no entry is near (kLostWord:
-// neither has room).
+// Entry of a leaf in which something is counted, or -(g + 1) for slot g of the device table where no
+// entry is near (kLostWord: neither has room).
 __device__ __noinline__ int count_leaf_slow(uint32_t* tags, const MapView& m, unsigned long long key,
                                             uint32_t code, uint32_t epoch) {
   uint32_t h = count_home(code);
@@ -1624,11 +1627,12 @@ __global__ void __launch_bounds__(128) k_traverse_count(const __grid_constant__ 
         if (((volatile uint32_t*)s_tags)[e] == code) return (int)e;
         return count_leaf_slow(s_tags, m, tt.key(code), code, f.epoch);
       };
-      int leaf = find();
+      int leaf = kNoEntry;  // not looked up yet: only leaves with a label go into the map
       double t;
       for (;;) {
         t = fmin(fmin(t0, t1), t2);
         if (!(t <= r.len)) break;
+        if (leaf == kNoEntry) leaf = find();
         ++visits;
         if (leaf >= 0)
           atomicAdd(&s_counts[leaf * kCountLeafWords + (l & 127)], 1u << ((l >> 7) * 8));
@@ -1640,11 +1644,11 @@ __global__ void __launch_bounds__(128) k_traverse_count(const __grid_constant__ 
         l = (l & ~msk) | (vv & msk);
         if ((unsigned)vv > (unsigned)msk) {
           code += msk == 0x1C0 ? r.hs0 : (msk == 0x38 ? r.hs1 : r.hs2);
-          leaf = find();
+          leaf = kNoEntry;
         }
       }
       if (t < (double)f.max_time) {
-        end_leaf = leaf;
+        end_leaf = leaf == kNoEntry ? find() : leaf;
         end_l = l;
         ++visits;
       }

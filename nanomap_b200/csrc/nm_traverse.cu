@@ -398,7 +398,8 @@ struct MarchFrame {
   double inv_res;
   float far2, drop2;   // squared lengths (m): below far2 every length check passes with room,
                        // above drop2 the point is out of range
-  bool near[3];        // a first plane of the axis is closer than kNearPlane
+  bool near[3][2];     // the first plane is closer than kNearPlane: the set-up marks it, or sends the
+                       // ray to the DDA, and the march leaves it out
 };
 
 // Rays of a round.  Per axis and ray: `d` = end minus eye (m), `n` = planes to mark (bit 15: positive
@@ -461,7 +462,8 @@ __device__ __forceinline__ void march_frame(const FrameParams& f, MarchFrame& mf
     mf.fe[a] = f.eye[a] - v + kMagic;
     mf.first[a][0] = f.eye[a] - v;
     mf.first[a][1] = (v + 1.0) - f.eye[a];
-    mf.near[a] = f.eye[a] - v < (double)kNearPlane || (v + 1.0) - f.eye[a] < (double)kNearPlane;
+    mf.near[a][0] = f.eye[a] - v < (double)kNearPlane;
+    mf.near[a][1] = (v + 1.0) - f.eye[a] < (double)kNearPlane;
   } else if (a == 32) {
     mf.inv_res = 1.0 / f.res_d;
   } else if (a == 33) {
@@ -580,12 +582,12 @@ __device__ __forceinline__ void march_setup(const FrameParams& f, const MarchFra
   // First planes close to the eye: an eye near a lattice edge or corner crosses several of them
   // almost at once, which only their order decides.  (b, 0) comes before (a, 0) when
   // first_b / |d_b| < first_a / |d_a|; both zero: the higher axis first, as in the DDA.
-  if ((mf.near[0] | mf.near[1] | mf.near[2]) && live) {
+  if (live && (mf.near[0][d[0] > 0.0f] | mf.near[1][d[1] > 0.0f] | mf.near[2][d[2] > 0.0f])) {
     bool tie = false;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
+      if (!mf.near[a][d[a] > 0.0f] || n[a] <= 0) continue;
       const float fa = (float)mf.first[a][d[a] > 0.0f];
-      if (!(fa < kNearPlane) || n[a] <= 0) continue;
       int v[3];
       v[a] = d[a] > 0.0f ? 1 : -1;
       bool sure = true;
@@ -997,7 +999,7 @@ __device__ __forceinline__ void march_planes(const MarchFrame& mf, const TileTab
       }
       __syncwarp();
       // a first plane close to the eye was marked by the set-up
-      if (j == 0 && f0 < (double)kNearPlane) mask = 0u;
+      if (j == 0 && mf.near[a][s]) mask = 0u;
       mask |= __shfl_xor_sync(kFull, mask, 16);
       mask = (mask << 16) | (mask >> 16);
       march_write(a, tt, m, mask, s ? mf.v[a] + 1 + j : mf.v[a] - 1 - j,
@@ -1017,7 +1019,7 @@ __device__ __forceinline__ void march_planes(const MarchFrame& mf, const TileTab
         const double mc = (double)mr.d[c * mr.count + r] * inv;
         const double f0 = mf.first[a][s];
         // a first plane close to the eye was marked by the set-up
-        const int first = max((int)(entry >> 16), f0 < (double)kNearPlane ? 1 : 0);
+        const int first = max((int)(entry >> 16), mf.near[a][s] ? 1 : 0);
         if (march_outside(tt, m, a, s, mb, mc, f0, mf.fe[b], mf.fe[c], mf.v[a], mf.v[b], mf.v[c],
                           by8 ? first + (lane & 7) : first, by8 ? 8 : 1, n, epoch, plane)) {
           atomicOr(&ms.undecided[r >> 5], 1u << (r & 31));

@@ -1,0 +1,63 @@
+"""Labels of single frames against the CPU oracle, bit-identical, where a ray's first and last voxels are
+hard to tell: first planes almost at the eye, and ends almost at the maximum range.
+"""
+import numpy as np
+import pytest
+import torch
+
+from nanomap_b200 import _native as N
+from nanomap_b200 import api as A
+from oracle import oracle as O
+from tests.workloads import compare_labels, compare_maps, oracle_frame
+
+pytestmark = pytest.mark.gpu
+
+ROUNDINGS = [N.NM_ROUND_DOWN, N.NM_ROUND_NEAREST]
+
+
+def _check(ctx, pts, eye, res, rng_m, rounding):
+    """Inserts the records `pts` (h, w, 3), world offsets from the eye."""
+    h, w, _ = pts.shape
+    desc = A.sensor_desc(hres=w, vres=h, max_range=rng_m, explicit_log_odds=1, log_odds_hit=0.85,
+                         log_odds_miss=-0.4)
+    m, om = A.Map(ctx, A.map_desc(res=res, rounding=rounding)), O.Map(res, rounding=rounding)
+    rec = np.zeros((h, w, 4), np.float32)
+    rec[..., :3] = pts
+    pose = A.Pose(eye, (1.0, 0.0, 0.0, 0.0))
+    m.insert_points(A.Sensor(ctx, desc), pose, torch.from_numpy(rec).cuda(), w, h, 16,
+                    flags=N.NM_DEFER_INTEGRATE)
+    R, e, mt = oracle_frame(desc, pose, res, rounding)
+    om.insert(R, e, mt, desc.log_odds_hit, desc.log_odds_miss, rec[..., :3].reshape(-1, 3), keep_labels=True)
+    errs = compare_labels(m.export_labels(), om.labels())
+    assert not errs, "; ".join(errs[:4])
+    m.integrate()
+    errs = compare_maps(m.export(), om.export())
+    assert not errs, "; ".join(errs[:4])
+    st, ost = m.stats(), om.stats()
+    for k in ("visits", "rays", "unique_voxels"):
+        assert st[k] == ost[k], k
+    return e
+
+
+@pytest.mark.parametrize("rounding", ROUNDINGS)
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_first_plane_at_the_near_limit(ctx, rounding, axis):
+    """An eye whose distance to a plane is below the limit of close planes (1e-4f), by so little that
+    it rounds to it as a float."""
+    res, limit = 0.05, np.float32(1e-4)
+    p = np.float32(limit * np.float32(res))
+    for _ in range(40):
+        d = float(p) * (1.0 / float(np.float32(res)))
+        if d < float(limit) and np.float32(d) == limit:
+            break
+        p = np.nextafter(p, np.float32(0.0)) if d >= float(limit) else np.nextafter(p, np.float32(1.0))
+    else:
+        pytest.fail("no such eye")
+    eye = [0.137, -0.218, 0.391]
+    eye[axis] = float(p)
+    rng = np.random.default_rng(axis)
+    v = rng.normal(size=(16, 32, 3))
+    v[..., axis] = -np.abs(v[..., axis])
+    v *= rng.uniform(4.0, 9.5, (16, 32, 1)) / np.linalg.norm(v, axis=2, keepdims=True)
+    e = _check(ctx, v, tuple(eye), res, 10.0, rounding)
+    assert e[axis] < float(limit) and np.float32(e[axis]) == limit

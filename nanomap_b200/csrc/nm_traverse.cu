@@ -581,7 +581,8 @@ __device__ __forceinline__ void march_setup(const FrameParams& f, const MarchFra
 
   // First planes close to the eye: an eye near a lattice edge or corner crosses several of them
   // almost at once, which only their order decides.  (b, 0) comes before (a, 0) when
-  // first_b / |d_b| < first_a / |d_a|; both zero: the higher axis first, as in the DDA.
+  // first_b / |d_b| < first_a / |d_a|; both zero: the higher axis first, as in the DDA.  (The products
+  // below decide only while they are far from the denormals, where a factor has lost its precision.)
   if (live && (mf.near[0][d[0] > 0.0f] | mf.near[1][d[1] > 0.0f] | mf.near[2][d[2] > 0.0f])) {
     bool tie = false;
 #pragma unroll
@@ -599,9 +600,9 @@ __device__ __forceinline__ void march_setup(const FrameParams& f, const MarchFra
         const float fb = (float)mf.first[b][d[b] > 0.0f];
         const float x = fb * fabsf(d[a]), y = fa * fabsf(d[b]);
         bool before = y > x;
-        if (fa == 0.0f && fb == 0.0f)
+        if (mf.first[a][d[a] > 0.0f] == 0.0 && mf.first[b][d[b] > 0.0f] == 0.0)
           before = b > a;
-        else if (!(fabsf(x - y) > 1e-5f * (x + y)) ||
+        else if (!(x + y > 1e-30f) || !(fabsf(x - y) > 1e-5f * (x + y)) ||
                  !(y < 0.99f * (x + fabsf(d[a]))))  // not so far that (b, 1) comes in question
           sure = false;
         if (before) v[b] = d[b] > 0.0f ? 1 : -1;

@@ -61,3 +61,21 @@ def test_first_plane_at_the_near_limit(ctx, rounding, axis):
     v *= rng.uniform(4.0, 9.5, (16, 32, 1)) / np.linalg.norm(v, axis=2, keepdims=True)
     e = _check(ctx, v, tuple(eye), res, 10.0, rounding)
     assert e[axis] < float(limit) and np.float32(e[axis]) == limit
+
+
+@pytest.mark.parametrize("rounding", ROUNDINGS)
+@pytest.mark.parametrize("units", [(1, 7), (7, 1), (11, 4)])
+def test_denormal_eye(ctx, rounding, units):
+    """An eye a few denormal floats from a lattice edge.  In voxels of 0.3 m its distances to the two planes
+    are no whole number of them: all rays run between the direction that crosses both planes at once and
+    the one that seems to when the distances are rounded to floats."""
+    res, unit = 0.3, float(np.float32(1.4e-45))
+    e = [units[i] * unit / float(np.float32(res)) for i in range(2)]
+    true, rounded = e[1] / e[0], float(np.float32(e[1])) / float(np.float32(e[0]))
+    rng = np.random.default_rng(units[0])
+    v = -np.ones((16, 32, 3))
+    v[..., 1] = -(true + (rounded - true) * rng.uniform(0.2, 0.8, (16, 32)))
+    v[..., 2] = rng.normal(size=(16, 32)) * true
+    v *= rng.uniform(40.0, 58.0, (16, 32, 1)) / np.linalg.norm(v, axis=2, keepdims=True)
+    e = _check(ctx, v, (units[0] * unit, units[1] * unit, 0.391), res, 60.0, rounding)
+    assert 0.0 < e[0] < 1e-42 and 0.0 < e[1] < 1e-42

@@ -79,3 +79,23 @@ def test_denormal_eye(ctx, rounding, units):
     v *= rng.uniform(40.0, 58.0, (16, 32, 1)) / np.linalg.norm(v, axis=2, keepdims=True)
     e = _check(ctx, v, (units[0] * unit, units[1] * unit, 0.391), res, 60.0, rounding)
     assert 0.0 < e[0] < 1e-42 and 0.0 < e[1] < 1e-42
+
+
+@pytest.mark.parametrize("rounding", ROUNDINGS)
+@pytest.mark.parametrize("eye", [(0.137, -0.218, 0.391), (0.05, -0.2, 1.0), (0.0, 0.0, 0.0)])
+@pytest.mark.parametrize("reach", [9.0, 50.0, 80.0, 130.0, 400.0])
+def test_ends_near_the_range(ctx, rounding, eye, reach):
+    """Rays that end within three voxels of the range, or leave their end voxel there (a hit only when that
+    crossing comes before the range): walked tiles up to 80 voxels, marched ones from 130 on; axis-aligned
+    and diagonal rays among them, and ends up to 1e-6 voxels from the range."""
+    res = 0.05
+    rng = np.random.default_rng(int(reach))
+    d = rng.normal(size=(32, 32, 3))
+    d[:4] = np.eye(3)[rng.integers(0, 3, (4, 32))] * rng.choice([-1.0, 1.0], (4, 32, 1))
+    d[4:6] = np.sign(rng.normal(size=(2, 32, 3)))
+    d[6, :, 2] = 0.0
+    d /= np.linalg.norm(d, axis=2, keepdims=True)
+    r = reach - rng.uniform(0.0, 3.0, (32, 32, 1))
+    r[::5] = reach - 10.0 ** rng.uniform(-6.0, 0.0, (7, 32, 1))
+    r[1::5] = rng.uniform(1.0, reach, (7, 32, 1))
+    _check(ctx, d * r * res, eye, res, reach * res, rounding)

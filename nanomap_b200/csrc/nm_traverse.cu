@@ -26,9 +26,9 @@
 // bit.  The DDA's crossing times carry an absolute error below 2e-9 voxels over the longest ray (4000
 // rounded adds of up to 2^-42 each), so wherever the exact line stays further from the deciding
 // lattice plane than that and than the march's own arithmetic can be off, both choose the same
-// voxel.  A ray with any coordinate closer than 1e-8 voxels, or within two voxels of the maximum
-// range, or whose last crossing is as close to a tie, is walked by the DDA itself (setup_ray,
-// walk_ray).  walk_counted takes its number of steps from the same test.
+// voxel.  A ray with any coordinate closer than 1e-8 voxels, or whose last crossing is as close to a
+// tie, or whose length or last time is as close to the maximum range, is walked by the DDA itself
+// (setup_ray, walk_ray).  walk_counted takes its number of steps from the same test.
 //
 // Leaves are named by a leaf code lx*2^20 + ly*2^10 + lz (mod 2^32) relative to the eye's leaf,
 // one-to-one over every leaf a frame can reach while max_range / res stays below kNarrowMaxTime
@@ -399,8 +399,9 @@ struct MarchFrame {
   double first[3][2];  // distance to the first plane crossed
   int v[3];            // the eye's voxel
   double inv_res;
-  float far2, drop2;   // squared lengths (m): below far2 every length check passes with room,
-                       // above drop2 the point is out of range
+  // squared lengths (m): below far2 a ray leaves its end voxel before the maximum range, below sure2
+  // it ends before it, above drop2 the point is out of range
+  float far2, sure2, drop2;
   bool near[3][2];     // the first plane is closer than kNearPlane: the set-up marks it, or sends the
                        // ray to the DDA, and the march leaves it out
 };
@@ -473,6 +474,7 @@ __device__ __forceinline__ void march_frame(const FrameParams& f, MarchFrame& mf
     // a ray of this length leaves its end voxel (2 voxels across at most) before max_time
     const double reach = (double)f.max_time * f.res_d, far = reach - 2.0 * f.res_d;
     mf.far2 = far > 0.0 ? (float)(far * far * (1.0 - 1e-5)) : 0.0f;
+    mf.sure2 = (float)(reach * reach * (1.0 - 1e-5));
     mf.drop2 = (float)(reach * reach * (1.0 + 1e-5));
   }
 }
@@ -534,7 +536,7 @@ __device__ __forceinline__ void march_setup(const FrameParams& f, const MarchFra
   d[0] = d[1] = d[2] = 0.0f;
   n[0] = n[1] = n[2] = 0;
   bool walk = false;  // the DDA decides this ray
-  bool live = false;
+  bool live = false, hit = true;
   int total = 0;
   if (ok) {
     const float* R = f.R;
@@ -544,7 +546,7 @@ __device__ __forceinline__ void march_setup(const FrameParams& f, const MarchFra
                      A::fmul(R[3 * a + 2], p[2]));
     const float len2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
     if (len2 <= mf.drop2) {  // (NaN and Inf fall out here)
-      live = len2 < mf.far2 && len2 > 1e-13f;
+      live = len2 < mf.sure2 && len2 > 1e-13f;
       walk = !live;
     }
     if (live) {
@@ -571,8 +573,23 @@ __device__ __forceinline__ void march_setup(const FrameParams& f, const MarchFra
         }
       }
       total = n[0] + n[1] + n[2];
+      // Near the range a ray's end voxel is a hit only if the crossing that leaves it comes before the
+      // range.  (The DDA's times are within 2e-9 of the exact line's.  With all such rays left to the DDA
+      // each made its unit wait for one walk of full length: 640x480 at 10 m with 0.1 % of the rays
+      // ending there 124 -> 113.5 us, voxel-filtered 104 -> 84, a 64x1024 spinning sensor's at 20 m
+      // 71.5 -> 62.3.)
+      if (!(len2 < mf.far2)) {
+        const double dx = d[0], dy = d[1], dz = d[2], len = sqrt(dx * dx + dy * dy + dz * dz);
+        double t = DBL_MAX;
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          if (d[a] != 0.0f)
+            t = fmin(t, (mf.first[a][d[a] > 0.0f] + (double)n[a]) * (len / fabs((double)d[a])));
+        hit = t < (double)f.max_time;
+        walk |= fabs(t - (double)f.max_time) < 1e-8;
+      }
       live = !walk;
-      // the voxel entered by the last crossing is the end voxel: a hit, not a miss
+      // the voxel entered by the last crossing is the end voxel: no miss
 #pragma unroll
       for (int a = 0; a < 3; ++a) n[a] -= last == a ? 1 : 0;
     }
@@ -624,9 +641,10 @@ __device__ __forceinline__ void march_setup(const FrameParams& f, const MarchFra
   }
 
   if (live) {
-    visits += (uint32_t)total + 1u;
+    visits += (uint32_t)total + (hit ? 1u : 0u);
     rays += 1u;
-    // hit label of the end voxel
+  }
+  if (live && hit) {  // hit label of the end voxel
     const int x = mf.v[0] + end[0], y = mf.v[1] + end[1], z = mf.v[2] + end[2];
     const int base = leaf_base(tt, m, tt.code(x >> 3, y >> 3, z >> 3), f.epoch, f.plane);
     const int l = local_index(x, y, z);

@@ -99,3 +99,19 @@ def test_ends_near_the_range(ctx, rounding, eye, reach):
     r[::5] = reach - 10.0 ** rng.uniform(-6.0, 0.0, (7, 32, 1))
     r[1::5] = rng.uniform(1.0, reach, (7, 32, 1))
     _check(ctx, d * r * res, eye, res, reach * res, rounding)
+
+
+@pytest.mark.parametrize("rounding", ROUNDINGS)
+@pytest.mark.parametrize("spread", [2e-4, 2e-2, 1.0])
+@pytest.mark.parametrize("reach", [1000.0, 2500.0, 3900.0])
+def test_long_reach(ctx, rounding, spread, reach):
+    """Up to 3900 voxels of reach: past the 2032 planes of a window (a beam narrow enough to stay in it, one
+    that leaves it early, and rays of all directions)."""
+    res = 0.005
+    rng = np.random.default_rng(int(reach))
+    d = np.array([0.7, -0.5, 0.51]) + spread * rng.normal(size=(8, 32, 3))
+    d[0, :6] = np.concatenate([np.eye(3), -np.eye(3)])
+    d[0, 6:9] = [[1, 1, 1], [1, -1, 0], [0, 1, -1]]
+    d /= np.linalg.norm(d, axis=2, keepdims=True)
+    r = rng.uniform(0.5 * reach, reach, (8, 32, 1))
+    _check(ctx, d * r * res, (0.0137, -0.0218, 0.391), res, reach * res, rounding)

@@ -113,9 +113,15 @@ int nm_map_values_copy(nm_map m, float* dst, uint64_t max_floats, uint64_t* n_fl
   if (max_floats < n) return fail(NM_ERR_ARG, "destination holds %llu floats, map needs %llu",
                                   (unsigned long long)max_floats, (unsigned long long)n);
   NM_CUDA(cudaSetDevice(m->ctx->device));
-  // this device's aligned memory takes the kernel that does not read empty slots
+  // This device's aligned memory takes the kernel that does not read empty slots, while the table is
+  // known to hold few enough leaves (it moves 3 lines for a full slot, the copy 2; a table near the size
+  // of L2 is copied faster).  us by the share of slots in use, 0.1 / 0.2 / 0.3 / 0.4, and the whole copy's:
+  // 2^16 slots 39 / 46 / 49 / 53, 44; 2^17 64 / 76 / 86 / 96, 84; 2^18 112 / 134 / 153 / 173, 168; 2^19 208 /
+  // 248 / 288 / 326, 330.
+  const uint64_t few = m->view.capacity / (m->view.capacity < (1u << 18) ? 6 : 3);
   cudaPointerAttributes at{};
-  if (((uintptr_t)dst & 15u) == 0 && cudaPointerGetAttributes(&at, dst) == cudaSuccess &&
+  if (((uintptr_t)dst & 15u) == 0 && m->known_leaves < few &&
+      cudaPointerGetAttributes(&at, dst) == cudaSuccess &&
       at.type == cudaMemoryTypeDevice && at.device == m->ctx->device) {
     NM_CUDA(nm::launch_values_copy(m->view, dst, m->ctx->sm_count, nm::pick(m->ctx, stream)));
     return NM_OK;

@@ -260,14 +260,14 @@ __global__ void __launch_bounds__(256) k_rehash(MapView from, MapView to, uint32
 }
 
 // The log-odds of every leaf to its slot's place in `dst` (16-byte aligned).  A warp reads the keys
-// of 32 slots at once and copies the used ones, a 2 KB line each.
-__global__ void __launch_bounds__(256) k_values_copy(MapView m, float4* dst) {
-  const int lane = threadIdx.x & 31;
+// of `group` slots (8, 16 or 32) at once and copies the used ones, a 2 KB line each.
+__global__ void __launch_bounds__(256) k_values_copy(MapView m, float4* dst, uint32_t group) {
+  const uint32_t lane = threadIdx.x & 31;
   const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
   const float4* src = reinterpret_cast<const float4*>(m.values);
-  for (uint32_t s0 = gw * 32u; s0 < m.capacity; s0 += nw * 32u) {  // capacity: a power of two >= 1024
-    unsigned used = __ballot_sync(kFull, m.keys[s0 + lane] != kEmptyKey);
+  for (uint32_t s0 = gw * group; s0 < m.capacity; s0 += nw * group) {  // capacity: a power of two >= 1024
+    unsigned used = __ballot_sync(kFull, lane < group && m.keys[s0 + (lane & (group - 1u))] != kEmptyKey);
     for (; used; used &= used - 1u) {
       const size_t o = (size_t)(s0 + __ffs(used) - 1) * (kLeafVoxels / 4) + lane;
 #pragma unroll
@@ -417,7 +417,7 @@ cudaError_t launch_export(const MapView& m, int32_t* origins, float* values, uin
 }
 
 // An empty slot's log-odds are zero by construction (its storage is cleared when the table is made,
-// and only leaves are written), and a table is at most half full and mostly far emptier: zeros
+// and only leaves are written), and a table is mostly far emptier than its limit of 7/8: zeros
 // everywhere, then the leaves.  Bound by the memset's writes: 1.07 GB (2^19 slots, 2858 leaves) in
 // 184 us against 338 us for a device copy, which also reads the zeros (197 us when one kernel
 // wrote both).  A small table is copied whole: 33 MB (2^14 slots) in 8 us against 10 us, the second
@@ -428,8 +428,13 @@ cudaError_t launch_values_copy(const MapView& m, float* dst, int sm_count, cudaS
                            cudaMemcpyDeviceToDevice, s);
   const cudaError_t e = cudaMemsetAsync(dst, 0, (size_t)m.capacity * kLeafVoxels * 4, s);
   if (e != cudaSuccess) return e;
-  const uint32_t blocks = std::min<uint32_t>(m.capacity / 256u, (uint32_t)sm_count * 8u);
-  k_values_copy<<<blocks, 256, 0, s>>>(m, reinterpret_cast<float4*>(dst));
+  // as many slots a warp as still leave half of the resident warps a group (2^16 slots, of which 0.3 hold
+  // a leaf, 70.5 us with 32 slots a warp, 48.9 with 8)
+  const uint32_t resident = (uint32_t)sm_count * 8u;
+  uint32_t group = 32u;
+  while (group > 8u && m.capacity / (group * 8u) < resident / 2u) group >>= 1;
+  const uint32_t blocks = std::min<uint32_t>(m.capacity / (group * 8u), resident);
+  k_values_copy<<<blocks, 256, 0, s>>>(m, reinterpret_cast<float4*>(dst), group);
   return cudaGetLastError();
 }
 

@@ -1055,6 +1055,20 @@ __device__ __forceinline__ void march_planes(const MarchFrame& mf, const TileTab
   }
 }
 
+// Adds a thread's counts to the map's counters (one update per warp).
+__device__ __forceinline__ void add_ray_counts(const MapView& m, uint32_t visits, uint32_t rays) {
+  unsigned long long vv = visits, rr = rays;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    vv += __shfl_xor_sync(kFull, vv, o);
+    rr += __shfl_xor_sync(kFull, rr, o);
+  }
+  if ((threadIdx.x & 31) == 0 && (vv | rr)) {
+    atomicAdd(&m.ctr->visits, vv);
+    atomicAdd(&m.ctr->rays, rr);
+  }
+}
+
 // Range bucket of a pixel for the tile's ray order: 0 = longest rays, kSortBuckets - 1 =
 // shortest and rays without a return.
 // `qs` = kSortBuckets / max_range (metres): the bucket is the range's fraction of max range.
@@ -1382,16 +1396,7 @@ __device__ __forceinline__ void traverse_body(const TickWork<MaxF>& work, const 
     __syncthreads();
   }
 
-  unsigned long long vv = visits, rr = rays;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    vv += __shfl_xor_sync(kFull, vv, o);
-    rr += __shfl_xor_sync(kFull, rr, o);
-  }
-  if (lane == 0 && (vv | rr)) {
-    atomicAdd(&m.ctr->visits, vv);
-    atomicAdd(&m.ctr->rays, rr);
-  }
+  add_ray_counts(m, visits, rays);
 }
 
 // ---- tile order (longest walks first) --------------------------------------------------------
@@ -1570,12 +1575,38 @@ struct CountEmit {
   }
 };
 
+// Table-free: a thread per ray of 16 x 16 pixels (8 x 4 a warp), a look-up per leaf change and an atomic per
+// group of lanes that are in the same voxel.  For reaches past the leaf codes', and for large images: with
+// thousands of CTAs what counts is their throughput, and a table's clearing and copying out, with 4 CTAs a
+// SM for it, costs more than it saves.  us a frame, table / table-free: 640x480 at 10 m and 0.05 m (2400 tiles
+// of 16 x 8) 127 / 143, 848x480 at 8 m and 0.04 m (3180) 165 / 168, 1280x720 at 6 m and 0.1 m (7200) 174 / 110,
+// at 15 m and 0.02 m 787 / 663, 1920x1080 at 5 m and 0.05 m (16200) 579 / 338.
+template <int RM>
+__global__ void __launch_bounds__(256) k_traverse_count_free(const __grid_constant__ FrameParams f,
+                                                             MapView m, int tiles_x) {
+  const int tid = threadIdx.x, tile = blockIdx.x;
+  const int warp = tid >> 5, lane = tid & 31;
+  const int px = (tile % tiles_x) * 16 + (warp & 1) * 8 + (lane & 7);
+  const int py = (tile / tiles_x) * 16 + (warp >> 1) * 4 + (lane >> 3);
+  uint32_t visits = 0, rays = 0;
+  float p[3];
+  if (px < f.width && py < f.height && pixel_point(f, px, py, p)) {
+    CountEmit em{&m, f.epoch, kEmptyKey, -1};
+    const int n = trace_point<RM>(f, p[0], p[1], p[2], em);
+    if (n >= 0) {
+      visits = (uint32_t)n;
+      rays = 1;
+    }
+  }
+  add_ray_counts(m, visits, rays);
+}
 
 // A CTA takes 16 x 8 pixels, and its rays' misses are counted in shared memory: a table of leaves by
 // code (relative to the eye's leaf), with a byte per voxel, which 128 rays that each visit a voxel
 // at most once cannot overflow.  A leaf's voxels then go to the device counters in one coalesced
-// pass, and a leaf is looked up there once per CTA.  Bound before by match, device atomic and probe in
-// every step: 317x239 pixels at 5 m and 0.05 m 75 us a frame, 42.5 us now (of 592 CTAs all are resident; the longest rays bound it).
+// pass, and a leaf is looked up there once per CTA.  317x239 pixels at 5 m and 0.05 m 42 us a frame (of 592
+// CTAs all are resident; the longest rays bound it), with match, device atomic and probe in every step 80.
+// A CTA whose rays fan out over more leaves than pay for the table (count_extent) does it that way.
 constexpr int kCountLeaves = 104;                      // 4 CTAs a SM
 constexpr int kCountLeafWords = kLeafVoxels / 4;       // voxel l: byte l >> 7 of word l & 127, so
                                                        // neighbours lie in different words
@@ -1584,23 +1615,52 @@ constexpr size_t kCountBytes = (size_t)kCountLeaves * kCountLeafWords * 4;
 // A leaf that the walk has entered and not looked up.  (No entry, slot or lost leaf has this number.)
 constexpr int kNoEntry = INT_MIN + 1;
 
-__device__ __forceinline__ uint32_t count_home(uint32_t code) {
-  return __umulhi(code * 0x9E3779B1u, (uint32_t)kCountLeaves);
+// Buckets of four tags, read with one load: a leaf is at its home place or, where others hold that, at the
+// first place that was free in the rest of its bucket and then in the next two.  So the look-up of a leaf
+// that finds no room ends after three loads; with up to 24 single ones 320x240 pixels at 5 m and 0.01 m
+// (500 voxels of reach) took 930 us, 570 now and 606 without a table.
+constexpr uint32_t kCountBuckets = kCountLeaves / 4, kCountNear = 3;
+
+__device__ __forceinline__ uint4 count_bucket(const uint32_t* tags, uint32_t b) {
+  uint4 t;
+  asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(t.x), "=r"(t.y), "=r"(t.z), "=r"(t.w)
+               : "r"((uint32_t)__cvta_generic_to_shared(tags + 4 * b)));
+  return t;
 }
 
-// Entry of a leaf in which something is counted, or -(g + 1) for slot g of the device table where no
-// entry is near (kLostWord: neither has room).
+// Place of `code` in a bucket, -1 where it is not.
+__device__ __forceinline__ int count_place(const uint4& t, uint32_t code) {
+  return t.x == code ? 0 : (t.y == code ? 1 : (t.z == code ? 2 : (t.w == code ? 3 : -1)));
+}
+
+// Entry of a leaf in which something is counted, or, where its buckets are full, -(g + 1) for slot g of the
+// device table (kLostWord: no room there either).
 __device__ __noinline__ int count_leaf_slow(uint32_t* tags, const MapView& m, unsigned long long key,
-                                            uint32_t code, uint32_t epoch) {
-  uint32_t h = count_home(code);
-  for (int i = 0; i < 24; ++i) {
-    const uint32_t k = ((volatile uint32_t*)tags)[h];
-    if (k == code) return (int)h;
-    if (k == kNoLeaf) {
-      const uint32_t old = atomicCAS(&tags[h], kNoLeaf, code);
-      if (old == kNoLeaf || old == code) return (int)h;
+                                            uint32_t code, uint32_t home, uint32_t epoch) {
+  auto bucket = [&](uint32_t q) {
+    const uint32_t b = (home >> 2) + q;
+    return b < kCountBuckets ? b : b - kCountBuckets;
+  };
+  for (uint32_t i = 0; i < 4u * kCountNear; ++i) {
+    if (i == 2u) {  // both first places are others': the rest at once
+      bool room = false;
+#pragma unroll
+      for (uint32_t q = 0; q < kCountNear; ++q) {
+        const uint4 t = count_bucket(tags, bucket(q));
+        const int at = count_place(t, code);
+        if (at >= 0) return (int)(4u * bucket(q)) + at;
+        room |= count_place(t, kNoLeaf) >= 0;
+      }
+      if (!room) break;
     }
-    h = h + 1 == kCountLeaves ? 0 : h + 1;
+    const uint32_t e = 4u * bucket(i >> 2) + ((i < 4u ? home + i : i) & 3u);
+    uint32_t k = ((volatile uint32_t*)tags)[e];
+    if (k == kNoLeaf) {
+      k = atomicCAS(&tags[e], kNoLeaf, code);
+      if (k == kNoLeaf) return (int)e;
+    }
+    if (k == code) return (int)e;
   }
   const int g = map_find_or_insert(m, key);
   if (g < 0) return kLostWord;
@@ -1608,14 +1668,85 @@ __device__ __noinline__ int count_leaf_slow(uint32_t* tags, const MapView& m, un
   return -(g + 1);
 }
 
+struct CountExtent {
+  uint32_t lo[4][3], hi[4][3];  // per warp and axis: least and greatest component of a unit direction
+  uint32_t len[4], n[4];        // sum of the lengths (leaves), rays
+};
+
+// Leaves that a CTA's rays fan out over, estimated from their mean length L (in leaves) and the two
+// widest spreads a, b of their directions: the integral of (1 + a t)(1 + b t) over [0, L].
+__device__ __forceinline__ float count_extent(const FrameParams& f, bool ok, const float p[3],
+                                              CountExtent& ext) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float len = sqrtf(p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {  // components moved to [1, 3]: floats in the order of their bits
+    const uint32_t u = __float_as_uint(2.0f + fminf(fmaxf(__fdividef(p[a], len), -1.0f), 1.0f));
+    const uint32_t lo = __reduce_min_sync(kFull, ok ? u : 0xFFFFFFFFu);
+    const uint32_t hi = __reduce_max_sync(kFull, ok ? u : 0u);
+    if (lane == 0) ext.lo[warp][a] = lo;
+    if (lane == 0) ext.hi[warp][a] = hi;
+  }
+  const float leaves = __fdividef(len, (float)f.res_d * 8.0f);
+  const uint32_t sum = __reduce_add_sync(kFull, ok ? (uint32_t)(fminf(leaves, 4096.0f) * 16.0f) : 0u);
+  const unsigned have = __ballot_sync(kFull, ok);
+  if (lane == 0) ext.len[warp] = sum;
+  if (lane == 0) ext.n[warp] = __popc(have);
+  __syncthreads();
+  float s[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    uint32_t lo = ext.lo[0][a], hi = ext.hi[0][a];
+#pragma unroll
+    for (int w = 1; w < 4; ++w) lo = min(lo, ext.lo[w][a]), hi = max(hi, ext.hi[w][a]);
+    s[a] = __uint_as_float(hi) - __uint_as_float(lo);
+  }
+  const float L = __fdividef((float)(ext.len[0] + ext.len[1] + ext.len[2] + ext.len[3]) * (1.0f / 16.0f),
+                             (float)(ext.n[0] + ext.n[1] + ext.n[2] + ext.n[3]));
+  const float least = fminf(fminf(s[0], s[1]), s[2]);
+  const float both = s[0] + s[1] + s[2] - least;  // a + b
+  const float a = fmaxf(fmaxf(s[0], s[1]), s[2]), b = both - a;
+  return L * (1.0f + L * (0.5f * both + L * a * b * (1.0f / 3.0f)));
+}
+
+// The limits of count_extent.  Beyond about the table's size the leaves without room cost what the others
+// gain: 160x120 pixels at 4 m and 0.02 m 191 us at 48, 134 at 96 and above; 200x150 at 2.5 m and 0.005 m (500
+// voxels of reach) 661 at 96, 719 without a limit; 40x30 at 10 m and 0.02 m 494 / 568.  Records packed by the
+// voxel filter come from several patches, and their box is far wider than the leaves they visit, the more
+// so the shorter they are: 317x239 at 5 m and 0.05 m (100 voxels) 93 us at 96, 69 at 192, 55 at 400 and above;
+// 1024 pixels in a row at 12 m and 0.05 m (240) 158 at 400, 114 at 1000; but a 512x32 spinning sensor at 60 m
+// and 0.05 m (1200) 181 at 400, 225 at 1000, 320x240 at 5 m and 0.01 m (500) 672 / 719, 1280x720 at 6 m and
+// 0.03 m 183 / 205.
+constexpr float kCountFan = 96.0f, kCountFanPacked = 1000.0f, kCountFanPackedLong = 400.0f;
+constexpr float kCountShort = 256.0f;    // voxels of reach
+constexpr int64_t kCountTiles = 4096;    // a large image has more tiles of 16 x 8
+
 template <int RM>
 __global__ void __launch_bounds__(128) k_traverse_count(const __grid_constant__ FrameParams f,
-                                                        MapView m, int tiles_x, int narrow) {
+                                                        MapView m, int tiles_x, float fan) {
   extern __shared__ uint4 s_raw[];
   uint32_t* s_counts = (uint32_t*)s_raw;
-  __shared__ uint32_t s_tags[kCountLeaves];
+  __shared__ __align__(16) uint32_t s_tags[kCountLeaves];
   __shared__ int s_slot[kCountLeaves];
+  __shared__ CountExtent s_ext;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tile = blockIdx.x;
+  // a warp's rays: a patch of 8 x 4 pixels
+  const int px = (tile % tiles_x) * 16 + (warp & 1) * 8 + (lane & 7);
+  const int py = (tile / tiles_x) * 8 + (warp >> 1) * 4 + (lane >> 3);
+  float p[3] = {0.0f, 0.0f, 0.0f};
+  Ray r;
+  const bool ok = px < f.width && py < f.height && pixel_point(f, px, py, p) && setup_ray<RM>(f, p, r);
+  if (!__syncthreads_or(ok)) return;
+  uint32_t visits = 0, rays = 0;
+  if (count_extent(f, ok, p, s_ext) > fan) {
+    if (ok) {
+      CountEmit em{&m, f.epoch, kEmptyKey, -1};
+      visits = (uint32_t)trace_point<RM>(f, p[0], p[1], p[2], em);
+      rays = 1;
+    }
+    add_ray_counts(m, visits, rays);
+    return;
+  }
   for (int i = tid; i < (int)(kCountBytes / 16); i += 128) s_raw[i] = make_uint4(0, 0, 0, 0);
   if (tid < kCountLeaves) s_tags[tid] = kNoLeaf;
   __syncthreads();
@@ -1623,59 +1754,44 @@ __global__ void __launch_bounds__(128) k_traverse_count(const __grid_constant__ 
   tt.elx = (int)floor(f.eye[0]) >> 3;
   tt.ely = (int)floor(f.eye[1]) >> 3;
   tt.elz = (int)floor(f.eye[2]) >> 3;
-  // a warp's rays: a patch of 8 x 4 pixels
-  const int px = (tile % tiles_x) * 16 + (warp & 1) * 8 + (lane & 7);
-  const int py = (tile / tiles_x) * 8 + (warp >> 1) * 4 + (lane >> 3);
-  uint32_t visits = 0, rays = 0;
   int end_leaf = kLostWord, end_l = 0;
-  float p[3];
-  if (px < f.width && py < f.height && pixel_point(f, px, py, p)) {
-    Ray r;
-    if (!narrow) {  // out of the codes' reach
-      CountEmit em{&m, f.epoch, kEmptyKey, -1};
-      const int n = trace_point<RM>(f, p[0], p[1], p[2], em);
-      if (n >= 0) {
-        visits = (uint32_t)n;
-        rays = 1;
+  if (ok) {
+    double t0 = r.t0, t1 = r.t1, t2 = r.t2;
+    int l = r.l;
+    uint32_t code = r.code;
+    auto find = [&]() -> int {
+      const uint32_t home = __umulhi(code * 0x9E3779B1u, (uint32_t)kCountLeaves);
+      if (((volatile uint32_t*)s_tags)[home] == code) return (int)home;
+      const uint32_t second = (home & ~3u) + ((home + 1u) & 3u);
+      if (((volatile uint32_t*)s_tags)[second] == code) return (int)second;
+      return count_leaf_slow(s_tags, m, tt.key(code), code, home, f.epoch);
+    };
+    int leaf = kNoEntry;  // not looked up yet: only leaves with a label go into the map
+    double t;
+    for (;;) {
+      t = fmin(fmin(t0, t1), t2);
+      if (!(t <= r.len)) break;
+      if (leaf == kNoEntry) leaf = find();
+      ++visits;
+      if (leaf >= 0)
+        atomicAdd(&s_counts[leaf * kCountLeafWords + (l & 127)], 1u << ((l >> 7) * 8));
+      else if (leaf != kLostWord)
+        add_one(m, (unsigned long long)(-leaf - 1) * 1024ull + 512u + (unsigned)l);
+      int msk, ds;
+      dda_step<RM>(t0, t1, t2, r.d0, r.d1, r.d2, r.ds0, r.ds1, r.ds2, msk, ds);
+      const int vv = (l & msk) + ds;
+      l = (l & ~msk) | (vv & msk);
+      if ((unsigned)vv > (unsigned)msk) {
+        code += msk == 0x1C0 ? r.hs0 : (msk == 0x38 ? r.hs1 : r.hs2);
+        leaf = kNoEntry;
       }
-    } else if (setup_ray<RM>(f, p, r)) {
-      double t0 = r.t0, t1 = r.t1, t2 = r.t2;
-      int l = r.l;
-      uint32_t code = r.code;
-      auto find = [&]() -> int {
-        uint32_t e = count_home(code);
-        if (((volatile uint32_t*)s_tags)[e] == code) return (int)e;
-        e = e + 1 == kCountLeaves ? 0 : e + 1;
-        if (((volatile uint32_t*)s_tags)[e] == code) return (int)e;
-        return count_leaf_slow(s_tags, m, tt.key(code), code, f.epoch);
-      };
-      int leaf = kNoEntry;  // not looked up yet: only leaves with a label go into the map
-      double t;
-      for (;;) {
-        t = fmin(fmin(t0, t1), t2);
-        if (!(t <= r.len)) break;
-        if (leaf == kNoEntry) leaf = find();
-        ++visits;
-        if (leaf >= 0)
-          atomicAdd(&s_counts[leaf * kCountLeafWords + (l & 127)], 1u << ((l >> 7) * 8));
-        else if (leaf != kLostWord)
-          add_one(m, (unsigned long long)(-leaf - 1) * 1024ull + 512u + (unsigned)l);
-        int msk, ds;
-        dda_step<RM>(t0, t1, t2, r.d0, r.d1, r.d2, r.ds0, r.ds1, r.ds2, msk, ds);
-        const int vv = (l & msk) + ds;
-        l = (l & ~msk) | (vv & msk);
-        if ((unsigned)vv > (unsigned)msk) {
-          code += msk == 0x1C0 ? r.hs0 : (msk == 0x38 ? r.hs1 : r.hs2);
-          leaf = kNoEntry;
-        }
-      }
-      if (t < (double)f.max_time) {
-        end_leaf = leaf == kNoEntry ? find() : leaf;
-        end_l = l;
-        ++visits;
-      }
-      rays = 1;
     }
+    if (t < (double)f.max_time) {
+      end_leaf = leaf == kNoEntry ? find() : leaf;
+      end_l = l;
+      ++visits;
+    }
+    rays = 1;
   }
   __syncthreads();
   for (int e = tid; e < kCountLeaves; e += 128) {
@@ -1707,16 +1823,7 @@ __global__ void __launch_bounds__(128) k_traverse_count(const __grid_constant__ 
       }
     }
   }
-  unsigned long long vv = visits, rr = rays;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    vv += __shfl_xor_sync(kFull, vv, o);
-    rr += __shfl_xor_sync(kFull, rr, o);
-  }
-  if (lane == 0 && (vv | rr)) {
-    atomicAdd(&m.ctr->visits, vv);
-    atomicAdd(&m.ctr->rays, rr);
-  }
+  add_ray_counts(m, visits, rays);
 }
 
 // Work list passed by value (single insert, one-shot tick).  MinB resident CTAs per SM: at 4 the
@@ -1866,14 +1973,21 @@ cudaError_t launch_traverse_labels(const TickWork<MaxF>& w, const MapView& m, in
 
 cudaError_t launch_traverse_counts(const FrameParams& f, const MapView& m, int rounding,
                                    cudaStream_t s) {
+  const bool down = rounding == NM_ROUND_DOWN, packed = f.input_kind == 2;
   const int tiles_x = (f.width + 15) / 16, tiles_y = (f.height + 7) / 8;
-  const int narrow = f.max_time < kNarrowMaxTime ? 1 : 0;
-  auto kernel = rounding == NM_ROUND_DOWN ? k_traverse_count<NM_ROUND_DOWN>
-                                          : k_traverse_count<NM_ROUND_NEAREST>;
+  const bool large = (int64_t)tiles_x * tiles_y > kCountTiles;
+  if (!(f.max_time < kNarrowMaxTime) || (large && !packed)) {
+    auto kernel = down ? k_traverse_count_free<NM_ROUND_DOWN> : k_traverse_count_free<NM_ROUND_NEAREST>;
+    kernel<<<tiles_x * ((f.height + 15) / 16), 256, 0, s>>>(f, m, tiles_x);
+    return cudaGetLastError();
+  }
+  const float fan = !packed ? kCountFan
+                            : (large || f.max_time > kCountShort ? kCountFanPackedLong : kCountFanPacked);
+  auto kernel = down ? k_traverse_count<NM_ROUND_DOWN> : k_traverse_count<NM_ROUND_NEAREST>;
   const cudaError_t e =
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountBytes);
   if (e != cudaSuccess) return e;
-  kernel<<<tiles_x * tiles_y, 128, kCountBytes, s>>>(f, m, tiles_x, narrow);
+  kernel<<<tiles_x * tiles_y, 128, kCountBytes, s>>>(f, m, tiles_x, fan);
   return cudaGetLastError();
 }
 

@@ -225,22 +225,16 @@ __device__ __forceinline__ void walk(const MapView& m, const float* __restrict__
   }
 }
 
-// Expected depth in index units (integral of the transmittance over [0, t_max]), FP32.  With
-// `entry_step` given, also the mean, over where the ray ends, of the voxel step along the axis
-// it entered the ending voxel across (1 / |d_a|, index units): the depth the ray covers from
-// one face of that voxel to the opposite one.
+// Expected depth in index units (integral of the transmittance over [0, t_max]), FP32.
 __device__ __forceinline__ float expected_index_depth(const DepthParams& p, const MapView& m,
                                                       const float* vals, const double d[3],
-                                                      float* t1_out, uint32_t* visits,
-                                                      float* entry_step = nullptr) {
+                                                      float* t1_out, uint32_t* visits) {
   DensityCache dc;
-  float T = 1.0f, acc = 0.0f, W = 0.0f;
+  float T = 1.0f, acc = 0.0f;
   double t1 = p.t_max;
   bool first = true;
   uint32_t n = 0;
-  const float step[3] = {(float)(1.0 / fabs(d[0])), (float)(1.0 / fabs(d[1])),
-                         (float)(1.0 / fabs(d[2]))};
-  walk<true>(m, vals, p.eye, d, p.t_max, [&](int, int, float L, double t_in, int a_in, double t_out) {
+  walk<true>(m, vals, p.eye, d, p.t_max, [&](int, int, float L, double t_in, int, double t_out) {
     ++n;
     dc.at(p, L);
     const float sg = dc.sg;
@@ -252,13 +246,11 @@ __device__ __forceinline__ float expected_index_depth(const DepthParams& p, cons
     float len;
     const float em1 = segment(sg, Dk, sg * Dk, &len);
     acc += T * len;
-    if (entry_step) W -= T * em1 * step[a_in];
     T *= 1.0f + em1;
     return T >= kStopTransmittance;
   });
   *t1_out = (float)t1;
   *visits += n;
-  if (entry_step) *entry_step = T < 1.0f ? W / (1.0f - T) : 0.0f;
   return (float)t1 + acc;
 }
 

@@ -76,18 +76,6 @@ __device__ __forceinline__ int map_find_or_insert(const MapView& m, unsigned lon
   return -1;
 }
 
-__device__ __forceinline__ int map_find(const MapView& m, unsigned long long key) {
-  uint32_t h = hash_key(key) & m.mask;
-  const uint32_t limit = m.capacity < kMaxProbe ? m.capacity : kMaxProbe;
-  for (uint32_t probe = 0; probe < limit; ++probe) {
-    const unsigned long long k = __ldcg(&m.keys[h]);
-    if (k == key) return (int)h;
-    if (k == kEmptyKey) return -1;
-    h = (h + 1) & m.mask;
-  }
-  return -1;
-}
-
 // Put `slot` on the touched list once per epoch; record the label plane for batched ticks.
 __device__ __forceinline__ void mark_touched(const MapView& m, int slot, uint32_t epoch,
                                              int plane) {
@@ -98,23 +86,6 @@ __device__ __forceinline__ void mark_touched(const MapView& m, int slot, uint32_
       m.touched[i] = (uint32_t)slot;
     }
   }
-}
-
-// Shared-memory leaf table of one CTA: `smask + 1` entries of (key, 32 label words).
-__device__ __forceinline__ int smem_find_or_insert(unsigned long long* s_keys, uint32_t smask,
-                                                   unsigned long long key) {
-  uint32_t h = hash_key(key) & smask;
-  const uint32_t limit = (smask + 1) < 32u ? (smask + 1) : 32u;
-  for (uint32_t i = 0; i < limit; ++i) {
-    const unsigned long long k = ((volatile unsigned long long*)s_keys)[h];
-    if (k == key) return (int)h;
-    if (k == kEmptyKey) {
-      const unsigned long long old = atomicCAS(&s_keys[h], kEmptyKey, key);
-      if (old == kEmptyKey || old == key) return (int)h;
-    }
-    h = (h + 1) & smask;
-  }
-  return -1;
 }
 
 __device__ __forceinline__ int local_index(int x, int y, int z) {

@@ -221,8 +221,8 @@ cudaError_t launch_tile_order(const TickWork<MaxF>& w, TileOrderBuffers* b, cuda
 cudaError_t launch_tile_order_dev(const TickWork<kMaxTickFrames>* d_work, uint32_t total_tiles,
                                   TileOrderBuffers* b, cudaStream_t s);
 
-// Dynamic shared memory of one traversal CTA (leaf table, ray order, rendered ranges).
-size_t traverse_smem_bytes(int tile_w, int tile_h, uint32_t smask, bool render);
+// Dynamic shared memory of one traversal CTA (leaf table, and ray order or march).
+size_t traverse_smem_bytes(int tile_w, int tile_h, uint32_t smask);
 // Whether a frame fits the fused render + traversal (reach within the leaf code's range).
 bool traverse_render_fits(const FrameParams& f);
 cudaError_t prepare_traverse_dev(int tile_w, int tile_h, uint32_t smask, int rounding, bool wide);

@@ -1479,8 +1479,6 @@ __global__ void __launch_bounds__(kOrderThreads) k_tile_order_dev(const TickWork
   tile_order_body<kMaxTickFrames>(*work, b);
 }
 
-int order_grid(uint32_t total_tiles) { return (int)total_tiles; }
-
 // Label sink of the wide-frame kernel: device-table lookups on leaf changes, one atomic per
 // new label bit.
 struct WideEmit {
@@ -1913,10 +1911,9 @@ bool work_is_wide(const FrameParams* fr, int n) {
 
 }  // namespace
 
-size_t traverse_smem_bytes(int tile_w, int tile_h, uint32_t smask, bool render) {
+size_t traverse_smem_bytes(int tile_w, int tile_h, uint32_t smask) {
   const size_t nent = (size_t)smask + 1;
   const size_t nrays = (size_t)tile_w * tile_h;
-  (void)render;
   const size_t march = march_bytes((int)std::min<size_t>(kMarchRays, nrays / 4));
   return nent * (kLabelWords * 4 + 4 + 4) + std::max<size_t>(nrays * (2 + 1 + 12), march);
 }
@@ -1939,7 +1936,7 @@ cudaError_t launch_traverse_labels(const TickWork<MaxF>& w, const MapView& m, in
       k_traverse_wide<NM_ROUND_NEAREST, MaxF><<<grid, block, 0, s>>>(w, m);
     return cudaGetLastError();
   }
-  const size_t smem = traverse_smem_bytes(w.tile_w, w.tile_h, w.smask, false);
+  const size_t smem = traverse_smem_bytes(w.tile_w, w.tile_h, w.smask);
   // Frames that do not fill 3 CTAs per SM gain more from the registers than from a fourth CTA:
   // 320x240 at 0.1 m (300 tiles) 22.0 against 24.3 us, 64x1024 spinning sensor at 20 m (256) 46.9
   // against 51.2, and voxel-filtered 640x480 frames (about 100 tiles of packed points, their
@@ -1997,7 +1994,7 @@ cudaError_t launch_traverse_render(const TickWork<1>& w, const MapView& m, const
                                    int rounding, cudaStream_t s) {
   if (!traverse_render_fits(w.fr[0])) return cudaErrorInvalidValue;
   const int block = min(kMarchThreads, w.tile_w * w.tile_h);
-  const size_t smem = traverse_smem_bytes(w.tile_w, w.tile_h, w.smask, true);
+  const size_t smem = traverse_smem_bytes(w.tile_w, w.tile_h, w.smask);
   const bool down = rounding == NM_ROUND_DOWN;
   const void* fn = down ? (const void*)k_traverse_render<NM_ROUND_DOWN>
                         : (const void*)k_traverse_render<NM_ROUND_NEAREST>;
@@ -2024,7 +2021,7 @@ const void* dev_kernel(int rounding, bool wide) {
 
 cudaError_t prepare_traverse_dev(int tile_w, int tile_h, uint32_t smask, int rounding, bool wide) {
   const int block = min(kMarchThreads, tile_w * tile_h);
-  const size_t smem = wide ? 0 : traverse_smem_bytes(tile_w, tile_h, smask, false);
+  const size_t smem = wide ? 0 : traverse_smem_bytes(tile_w, tile_h, smask);
   int grid = 0;
   return resident_grid(dev_kernel(rounding, wide), smem, block, &grid);
 }
@@ -2033,7 +2030,7 @@ cudaError_t launch_traverse_labels_dev(const TickWork<kMaxTickFrames>* d_work, u
                                        int tile_w, int tile_h, uint32_t smask, const MapView& m,
                                        int rounding, bool wide, cudaStream_t s) {
   const int block = min(kMarchThreads, tile_w * tile_h);
-  const size_t smem = wide ? 0 : traverse_smem_bytes(tile_w, tile_h, smask, false);
+  const size_t smem = wide ? 0 : traverse_smem_bytes(tile_w, tile_h, smask);
   int grid = 0;
   const cudaError_t e = resident_grid(dev_kernel(rounding, wide), smem, block, &grid);
   if (e != cudaSuccess) return e;
@@ -2112,7 +2109,7 @@ cudaError_t launch_tile_order(const TickWork<MaxF>& w, TileOrderBuffers* b, cuda
   if (w.total_tiles > b->capacity) return cudaErrorInvalidValue;
   cudaError_t e = clear_pending_counts(b, s);
   if (e != cudaSuccess) return e;
-  k_tile_order<MaxF><<<order_grid(w.total_tiles), kOrderThreads, 0, s>>>(w, *b);
+  k_tile_order<MaxF><<<(int)w.total_tiles, kOrderThreads, 0, s>>>(w, *b);
   e = cudaGetLastError();
   if (e == cudaSuccess) b->pending = true;
   return e;
@@ -2124,7 +2121,7 @@ cudaError_t launch_tile_order_dev(const TickWork<kMaxTickFrames>* d_work, uint32
   if (total_tiles > b->capacity) return cudaErrorInvalidValue;
   cudaError_t e = clear_pending_counts(b, s);
   if (e != cudaSuccess) return e;
-  k_tile_order_dev<<<order_grid(total_tiles), kOrderThreads, 0, s>>>(d_work, *b);
+  k_tile_order_dev<<<(int)total_tiles, kOrderThreads, 0, s>>>(d_work, *b);
   e = cudaGetLastError();
   if (e == cudaSuccess) b->pending = true;
   return e;

@@ -480,8 +480,9 @@ constexpr uint32_t kFilteredEntries = 512;  // leaf-table entries per tile of fi
 
 // Voxel filter of one frame: runs the filter on `f`'s input and rewrites `f` into the frame
 // of the filtered points (input kind 2: one record per occupied voxel, already rotated into
-// the world frame, packed in the input order of the voxels' first points, counted on the
-// device).  A traversal tile covers consecutive records: neighbouring rays.
+// the world frame, counted on the device, packed in the compaction order of the voxels' first
+// points within 1024 positions, these groups in any order).  A traversal tile covers consecutive
+// records: neighbouring rays.
 int apply_filter(nm_map m, nm::FrameParams& f, uint32_t flags, cudaStream_t s0) {
   const int64_t n = (int64_t)f.width * f.height;
   const int kb = nm::filter_key_bits(f.max_time);

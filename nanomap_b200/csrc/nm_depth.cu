@@ -137,8 +137,8 @@ __device__ __forceinline__ int depth_find(const MapView& m, unsigned long long k
 // current one is handed to f, so the load and the leaf look-up stay out of the chain (not for the
 // adjoint, whose gradient atomics bound it and whose registers are the tighter for it: 190 against
 // 185 us).  Times of one launch on the B200, before -> now: refinement step, 640x480 at 10 m and
-// 0.05 m, 140.5 -> 92 us (85 with kRefineBlocks), expected depth of
-// 1280x720 at 15 m and 0.02 m 872 -> 657 us, of 640x480 63.2 -> 56.6 us, its adjoint 185.8 -> 185.
+// 0.05 m, 140.7 -> 92 us (84.6 with kRefineBlocks), expected depth of
+// 1280x720 at 15 m and 0.02 m 868 -> 665 us, of 640x480 64.1 -> 60.1 us, its adjoint 185.4 -> 187.1.
 template <bool Ahead, class F>
 __device__ __forceinline__ void walk(const MapView& m, const float* __restrict__ vals,
                                      const double e[3], const double d[3], double t_max, F&& f) {
@@ -404,8 +404,8 @@ __global__ void __launch_bounds__(kDepthTile * kDepthTile) k_depth_forward(Depth
 }
 
 // `depth` (may be null): the forward's output at this pose and these values; the ray's
-// expected depth is then taken from it instead of a first replay.  16 CTAs per SM (64 registers): 185
-// us for a 640x480 adjoint given depths; 195 us at 79 registers.
+// expected depth is then taken from it instead of a first replay.  16 CTAs per SM (64 registers): 187
+// us for a 640x480 adjoint given depths; about 10 us more at 79 registers.
 __global__ void __launch_bounds__(kDepthTile * kDepthTile, 16) k_depth_backward(
     DepthParams p, MapView m, const float* vals, const float* grad_depth, const float* depth,
     float* grad_vals, double* partials) {
@@ -601,7 +601,7 @@ __device__ void rotate_left(const double phi[3], double R[9]) {
 // fixed order (deterministic); h[c] = sum of column c, on every thread.  Thread t adds rows t / 8,
 // t / 8 + 128, ... of column t % 8 (neighbouring threads read neighbouring words, four rows in
 // flight), then a shuffle tree and one over the warps.  Bound by the latency of its 10 dependent
-// loads: 40.7 -> 9 us in the refinement step's update and 27.7 -> 6 us after an adjoint, both for
+// loads: 43.5 -> 10 us in the refinement step's update and 28 -> 12 us after an adjoint, both for
 // the 4800 rows of a 640x480 image (one column at a time over 256 threads before).
 constexpr int kSumThreads = 1024;
 template <int N>

@@ -24,7 +24,7 @@
 //
 // The march's labels are those of the double-precision DDA under the map's rounding mode bit for
 // bit.  The DDA's crossing times carry an absolute error below 2e-9 voxels over the longest ray (4000
-// rounded adds of up to 2^-42 each), so wherever the exact line stays further from the deciding
+// rounded adds of at most 2^-41 each), so wherever the exact line stays further from the deciding
 // lattice plane than that and than the march's own arithmetic can be off, both choose the same
 // voxel.  A ray with any coordinate closer than 1e-8 voxels, or whose last crossing is as close to a
 // tie, or whose length or last time is as close to the maximum range, is walked by the DDA itself
@@ -331,7 +331,7 @@ __device__ __forceinline__ void dda_step(double& t0, double& t1, double& t2, dou
 // walk_ray for a ray whose number of crossings `n` is known: the loop counts down instead of comparing
 // the next crossing's time with the ray's length, and needs that time only at its end, so each
 // axis's time is advanced in place under a predicate.  Bound by issue; the 16-frame tick's
-// traversal took 856 us with walk_ray alone and takes 789 us.
+// traversal took 856 us with walk_ray alone and takes 783 us.
 template <int RM>
 __device__ __forceinline__ uint32_t walk_counted(const Ray& r, int n, const TileTable& tt,
                                                  const MapView& m, double max_time, uint32_t epoch,
@@ -903,9 +903,9 @@ __device__ __forceinline__ bool march_outside(const TileTable& tt, const MapView
 //
 // What bounds it: latency, at a third of the issue rate (33.5 M warp instructions for 14.7 M voxel
 // visits of one 640x480 frame against the walk's 42 M, but eight barriers a unit); so it pays where
-// the walk leaves SMs idle.  Traversal of one frame, before -> now (B200): 64x1024 spinning sensor
-// at 20 m and 0.05 m 116.5 -> 46.9 us, 1280x720 at 15 m and 0.02 m 1187 -> 414 us, voxel-filtered
-// 640x480 at 10 m and 0.05 m 82 -> 66 us, unfiltered 94.7 -> 84.5 us.
+// the walk leaves SMs idle.  Traversal of one frame, walk alone -> now (B200): 64x1024 spinning sensor
+// at 20 m and 0.05 m 114 -> 47.3 us, 1280x720 at 15 m and 0.02 m 1179 -> 410 us, voxel-filtered
+// 640x480 at 10 m and 0.05 m 83.6 -> 58.1 us, unfiltered 94.5 -> 82.3 us.
 __device__ __forceinline__ void march_planes(const MarchFrame& mf, const TileTable& tt,
                                              const MapView& m, const MarchRays& mr,
                                              MarchShared& ms, uint32_t epoch, int plane) {
@@ -1414,9 +1414,10 @@ constexpr float kSetupSteps = 8.0f;
 // walk is the cheaper way to label a tile of short rays while enough tiles keep the SMs busy;
 // what the march removes is the wait for the last long rays, which a frame of few tiles feels
 // sooner.  Traversal times (us) by this limit, one frame each: 64x1024 spinning sensor at 20 m
-// (256 tiles) 51 / 54 / 73 / 124 at 96 / 128 / 192 / never; 640x480 camera at 10 m (1200 tiles)
-// 91 / 88 / 93 / 99; 1280x720 at 0.02 m and 15 m (3600 tiles) 535 / 515 / 468 / 1134 (at 256:
-// 468); the 16-frame tick (20 K tiles) 1029 / 973 / 871 / 851.
+// (256 tiles) 47 / 48 / 60 / 113 at 96 / 128 / 192 / never; 640x480 camera at 10 m (1200 tiles)
+// 86 / 82 / 86 / 95, the same voxel-filtered (about 100 tiles with points) 58 / 62 / 72 / 75; 1280x720 at
+// 0.02 m and 15 m (3600 tiles) 523 / 493 / 427 / 1143 (at 256: 411); the 16-frame tick (20 K tiles)
+// 983 / 920 / 811 / 784.
 constexpr float kSplitSteps = 64.0f;
 constexpr float kSplitStepsPerTile = 32.0f / 592.0f;
 constexpr int kOrderThreads = 128;
@@ -1938,10 +1939,10 @@ cudaError_t launch_traverse_labels(const TickWork<MaxF>& w, const MapView& m, in
   }
   const size_t smem = traverse_smem_bytes(w.tile_w, w.tile_h, w.smask);
   // Frames that do not fill 3 CTAs per SM gain more from the registers than from a fourth CTA:
-  // 320x240 at 0.1 m (300 tiles) 22.0 against 24.3 us, 64x1024 spinning sensor at 20 m (256) 46.9
-  // against 51.2, and voxel-filtered 640x480 frames (about 100 tiles of packed points, their
-  // number known on the device only) 66.0 against 69.4; 640x480 (1200) 86.0 against 84.5,
-  // 1280x720 at 0.02 m (3600) 437 against 414.
+  // 320x240 at 0.1 m (300 tiles) 21.5 against 24.2 us, 64x1024 spinning sensor at 20 m (256) 47.4
+  // against 51.9, and voxel-filtered 640x480 frames (about 100 tiles of packed points, their
+  // number known on the device only) 57.9 against 59.8; 640x480 (1200) 84.8 against 82.3,
+  // 1280x720 at 0.02 m (3600) 435 against 412.
   const bool roomy = MaxF == 1 && (w.total_tiles <= 3u * 148u || w.fr[0].input_kind == 2);
   using Kernel = void (*)(TickWork<MaxF>, MapView);
   constexpr int kFew = MaxF == 1 ? 3 : 4;

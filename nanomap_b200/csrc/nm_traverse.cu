@@ -1603,8 +1603,8 @@ __global__ void __launch_bounds__(256) k_traverse_count_free(const __grid_consta
 // A CTA takes 16 x 8 pixels, and its rays' misses are counted in shared memory: a table of leaves by
 // code (relative to the eye's leaf), with a byte per voxel, which 128 rays that each visit a voxel
 // at most once cannot overflow.  A leaf's voxels then go to the device counters in one coalesced
-// pass, and a leaf is looked up there once per CTA.  317x239 pixels at 5 m and 0.05 m 42 us a frame (of 592
-// CTAs all are resident; the longest rays bound it), with match, device atomic and probe in every step 80.
+// pass, and a leaf is looked up there once per CTA.  317x239 pixels at 5 m and 0.05 m 42 us a frame (600 CTAs,
+// 592 resident at once; the longest rays bound it), with match, device atomic and probe in every step 80.
 // A CTA whose rays fan out over more leaves than pay for the table (count_extent) does it that way.
 constexpr int kCountLeaves = 104;                      // 4 CTAs a SM
 constexpr int kCountLeafWords = kLeafVoxels / 4;       // voxel l: byte l >> 7 of word l & 127, so

@@ -1713,11 +1713,12 @@ __device__ __forceinline__ float count_extent(const FrameParams& f, bool ok, con
 // voxels of reach) 661 at 96, 719 without a limit; 40x30 at 10 m and 0.02 m 494 / 568.  Records packed by the
 // voxel filter come from several patches, and their box is far wider than the leaves they visit, the more
 // so the shorter they are: 317x239 at 5 m and 0.05 m (100 voxels) 93 us at 96, 69 at 192, 55 at 400 and above;
-// 1024 pixels in a row at 12 m and 0.05 m (240) 158 at 400, 114 at 1000; but a 512x32 spinning sensor at 60 m
-// and 0.05 m (1200) 181 at 400, 225 at 1000, 320x240 at 5 m and 0.01 m (500) 672 / 719, 1280x720 at 6 m and
-// 0.03 m 183 / 205.
-constexpr float kCountFan = 96.0f, kCountFanPacked = 1000.0f, kCountFanPackedLong = 400.0f;
-constexpr float kCountShort = 256.0f;    // voxels of reach
+// 1024 pixels in a row at 12 m and 0.05 m (240) 158 at 400, 114 at 1000; a 64x1024 spinning sensor at 20 m and
+// 0.05 m (400) 189 / 170.  Far rays differ: 320x240 at 5 m and 0.01 m (500) 617 at 192, 672 at 400, 719 at 1000,
+// 1280x720 at 15 m and 0.02 m (750) 494 / 526 / 547, 40x30 at 10 m and 0.02 m (500) 382 / 424 / 473.  Large images
+// of short reach: 1280x720 at 6 m and 0.03 m 183 at 400, 205 at 1000; 1920x1080 at 5 m and 0.05 m 67 at 192 and above.
+constexpr float kCountFan = 96.0f, kCountFanPacked = 1000.0f, kCountFanLarge = 400.0f, kCountFanFar = 192.0f;
+constexpr float kCountFar = 420.0f;      // voxels of reach
 constexpr int64_t kCountTiles = 4096;    // a large image has more tiles of 16 x 8
 
 template <int RM>
@@ -1979,8 +1980,10 @@ cudaError_t launch_traverse_counts(const FrameParams& f, const MapView& m, int r
     kernel<<<tiles_x * ((f.height + 15) / 16), 256, 0, s>>>(f, m, tiles_x);
     return cudaGetLastError();
   }
-  const float fan = !packed ? kCountFan
-                            : (large || f.max_time > kCountShort ? kCountFanPackedLong : kCountFanPacked);
+  const float fan = !packed                  ? kCountFan
+                    : f.max_time > kCountFar ? kCountFanFar
+                    : large                  ? kCountFanLarge
+                                             : kCountFanPacked;
   auto kernel = down ? k_traverse_count<NM_ROUND_DOWN> : k_traverse_count<NM_ROUND_NEAREST>;
   const cudaError_t e =
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountBytes);
